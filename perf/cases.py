@@ -357,7 +357,9 @@ def _scene_of(case, seed):
 
 # ------------------------------------------------------------------- prepare
 def prepare(case, seed):
-    return globals()["_prepare_" + case["kind"]](case, seed)
+    state = globals()["_prepare_" + case["kind"]](case, seed)
+    torch.cuda.synchronize()  # the handle works on a stream of its own
+    return state
 
 
 def run(state):
