@@ -19,6 +19,12 @@
 // then the backward substitution L^T x = y, right-looking by block rows:
 //   trsv_bwd(k): x_k = L_kk^-T y_k; y_j -= L_kj^T x_k for j < k.
 // A non-positive pivot sets *flag (LINEAR_SOLVER_FAILURE in ceres terms).
+// That is the FP32 path; the FP64 path has its own kernels for the panel and
+// the trailing update (k_panel64, k_syrk_split) and shares the backward
+// substitution.
+#include <cuda_fp16.h>
+#include <math_constants.h>
+
 #include <type_traits>
 
 #include "gbba_internal.h"
@@ -91,9 +97,8 @@ __device__ __forceinline__ void load_tile(T (*dst)[NB + 1], const T* __restrict_
 // Reciprocal of a pivot.  Single precision uses the fast hardware reciprocal
 // (__fdividef, within 2 ulp for normal pivots): it sits on the elimination's
 // critical path, and the FP32 factor only feeds LM steps whose acceptance is
-// decided on the FP64 cost.  Double precision divides exactly.
+// decided on the FP64 cost.
 __device__ __forceinline__ float pivot_rcp(float d) { return __fdividef(1.0f, d); }
-__device__ __forceinline__ double pivot_rcp(double d) { return 1.0 / d; }
 
 // Factor the diagonal tile: S_kk = L L^T (written back into S's lower
 // triangle, zeros above), L^-1 (into Linv_all), and y_k = L^-1 b_k.
@@ -655,6 +660,530 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ S, int64
                                 (part[tid] + part[NB + tid] + part[2 * NB + tid] + part[3 * NB + tid]);
 }
 
+// ---------------------------------------------------------------- FP64 factorisation
+// GB300 issues two FP64 FMAs a clock per multiprocessor, so in FP64 a 64 x 64
+// x 64 tile product takes 66 us on one SM.  The FP64 path therefore
+//   - splits a panel over all SMs (k_panel64: the diagonal tile factored by
+//     every CTA, at no cost in time, with 16 rows of the panel per CTA);
+//   - keeps the trailing update off the FP64 pipe (k_syrk_split): the products
+//     are formed exactly on the tensor cores from FP16 digits.
+// Factorisation and solve, against 64 x 64 tiles on the FP64 pipe: n = 114
+// 0.14 ms (0.40), n = 1,806 2.2 ms (7.9), n = 2,388 3.2 ms (11.7), n = 5,988
+// 17.4 ms (81.5); backward error the same (5.6e-16 at n = 2,388).
+//
+// Digits (error-free transformation of Ozaki, Ogita, Oishi and Rump, "Error-
+// free transformations of matrix multiplication", 2012): row i of the panel is
+// scaled by 2^e_i, its largest |l_ik| 2^e_i in [1/2, 1), and rounded to 62
+// fractional bits, q = sum_p d_p 2^(56 - 8 p) with eight balanced digits
+// |d_p| <= 128.  The digit products of equal weight p + q = g, g = 0..7, are
+// summed in one FP32 accumulator each: at most 8 products of 64 terms of at
+// most 2^14, so every partial sum is an integer of at most 2^23, exact in
+// FP32.  The eight sums make a 62-bit integer with integer arithmetic; what is
+// left out is about 2^-59 max_k |l_ik| max_k |l_jk| per panel, less than the
+// rounding of 64 FP64 FMAs.
+constexpr int kDigits = 8;
+constexpr int kDigitTile = 64 * 64;                            // one digit of a 64 x 64 tile (8 KB of FP16)
+constexpr size_t kTileDigitBytes = (size_t)kDigits * kDigitTile * 2;
+
+// 1 / d from the hardware's approximate reciprocal r: with e = 1 - d r, the
+// next terms of the geometric series 1 / d = r (1 + e + e^2 + ...) (Newton's
+// iteration of third order).
+__device__ __forceinline__ double rcp_series(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+// s = sqrt(d) and r = 1 / s: two of Newton's steps y += y (1 - d y^2) / 2 from
+// the hardware's approximation of 1 / sqrt(d), then s = d y and r = y with a
+// last step each, so that s r = 1 to rounding.
+__device__ __forceinline__ void sqrt_newton(double d, double& s, double& r) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const double e = fma(-d * y, y, 1.0);
+    y = fma(0.5 * y, e, y);
+  }
+  s = d * y;
+  s = fma(0.5 * y, fma(-s, s, d), s);
+  r = fma(y, fma(-s, y, 1.0), y);
+}
+__device__ __forceinline__ bool positive_finite(double d) {  // on the bits: FP64 comparisons run on the FP64 pipe
+  const unsigned hi = (unsigned)__double2hiint(d);
+  return hi < 0x7ff00000u && (hi | (unsigned)__double2loint(d)) != 0u;
+}
+
+// Panel kb: [L_kk; L_ik] of the diagonal tile and of this CTA's rows below it,
+// y_kb = L_kk^-1 b_kb, b_i -= L_ik y_kb and the digits of the rows.  L_kk with
+// its diagonal 16 x 16 blocks inverted goes to the tile's place in Linv, y_kb
+// to y: S_kk and b_kb stay as they are, other CTAs may still have to read them.  CTA j holds the rows
+// row0 + j R .. + R - 1 (row0 = 64 (kb + 1), R a multiple of 16; the grid has
+// at least one CTA, which may hold no rows) under a copy of the diagonal tile
+// and the row b_kb^T, and factors them together, 16 columns at a time:
+//   1. warps 0..3, one per scheduler (each holds a quarter of the SM's FP64
+//      lanes): the 16 x 16 diagonal block, LDL^T with the row operations
+//      applied to an identity block (its inverse).  Of the 16 columns l at
+//      pivot j, those right of j take the elimination of the block, the
+//      others that of the identity (its row j ends at column j); warp w holds
+//      columns w, w + 4, w + 8, w + 12 and passes a pivot's column on through
+//      shared memory, with one barrier of the four warps per pivot;
+//   2. L_ip = A_ip L_pp^-T for all rows below (a thread takes columns j and
+//      15 - j of a row: 17 products for the two, whatever j);
+//   3. A_il -= L_ip L_lp^T for the columns to the right.
+// Bound by FP64: about 100,000 FMAs for 16 rows (25 us at two a clock) and the
+// chain of 64 pivots (0.4 us each: reciprocal, multiplier, update).  nblk (4,
+// less in the last tile) is the number of 16-column blocks that hold
+// unknowns; the padding behind them is the identity already.
+// n = 2,388 (38 panels): 55 us a panel, against 199 + 134 us for a diagonal
+// kernel and one 64 x 64 tile per CTA.
+// 512 threads of 72 registers: no two CTAs of a panel share an SM (its FP64
+// pipe), and one of them leaves the registers for one CTA of the bulk update.
+constexpr int kPanelThreads = 512;
+constexpr int kPanelLd = 66;
+constexpr int kPanelMaxRows = 64;
+inline size_t panel64_smem(int R) { return sizeof(double) * ((size_t)(64 + R + 1) * kPanelLd + 4 * 16 * 18 + 256); }
+__global__ void __maxnreg__(72) k_panel64(double* __restrict__ S, int64_t ld, int kb, int R,
+                                                           int nblk, double* __restrict__ Linv_all,
+                                                           double* __restrict__ b, double* __restrict__ y,
+                                                           int32_t* __restrict__ ex, __half* __restrict__ digits,
+                                                           int* __restrict__ flag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* A = reinterpret_cast<double*>(smem_raw);         // rows 0..63 tile, 64..64+R-1 rows, 64+R: b^T
+  double* Li = A + (size_t)(64 + R + 1) * kPanelLd;        // [4][16][18] inverses of the diagonal blocks
+  double* cb = Li + 4 * 16 * 18;                           // [16][16] the pivots' columns
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t off = (int64_t)kb * NB;
+  const int64_t row0 = off + NB + (int64_t)blockIdx.x * R;
+  const int rows = (int)max((int64_t)0, min((int64_t)R, ld - row0));  // a multiple of 16
+  const int nr = 64 + rows;                                           // rows without b^T
+  for (int idx = tid; idx < nr * 32; idx += kPanelThreads) {
+    const int r = idx >> 5, c = (idx & 31) * 2;
+    const double2 v = *reinterpret_cast<const double2*>(S + (r < 64 ? off + r : row0 + r - 64) * ld + off + c);
+    *reinterpret_cast<double2*>(A + r * kPanelLd + c) = v;
+  }
+  double* yb = A + nr * kPanelLd;
+  if (tid < 64) yb[tid] = b[off + tid];
+  __syncthreads();
+  for (int p = 0; p < nblk; ++p) {
+    const int o = 16 * p;
+    double* Lp = Li + p * 16 * 18;
+    if (warp < 4) {
+      const int r = lane & 15;
+      const int l0 = warp + 4 * (lane >> 4), l1 = l0 + 8;  // this lane's columns of row r
+      double a0 = A[(o + r) * kPanelLd + o + l0], a1 = A[(o + r) * kPanelLd + o + l1];
+      double e0 = r == l0 ? 1.0 : 0.0, e1 = r == l1 ? 1.0 : 0.0;
+      if (l0 == 0) cb[r] = a0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const double* col = cb + 16 * j;
+        double d = col[j];
+        const double cr = col[r], c0 = col[l0], c1 = col[l1];
+        const double f0 = __shfl_sync(0xffffffffu, e0, j + (lane & 16)), f1 = __shfl_sync(0xffffffffu, e1, j + (lane & 16));
+        if (!positive_finite(d)) {  // non-positive, NaN or infinite pivot
+          d = 1.0;
+          if (tid == 0) {
+            cb[17 * j] = 1.0;
+            atomicExch(flag, 1);
+          }
+        }
+        const double m = r > j ? -cr * rcp_series(d) : 0.0;
+        // the next pivot's column first: the other warps wait for it
+        auto column = [&](int l, double& av, double& ev, double cl, double fl) {
+          const bool right = l > j;
+          const double v = fma(m, right ? cl : fl, right ? av : ev);
+          av = right ? v : av;
+          ev = right ? ev : v;
+          if (l == j + 1) cb[16 * (j + 1) + r] = av;
+        };
+        if (j + 1 < 8) {
+          column(l0, a0, e0, c0, f0);
+          column(l1, a1, e1, c1, f1);
+        } else {
+          column(l1, a1, e1, c1, f1);
+          column(l0, a0, e0, c0, f0);
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      // L_pp = L_u D^1/2, L_pp^-1 = D^-1/2 L_u^-1
+      double sd, rs;
+      sqrt_newton(cb[17 * r], sd, rs);
+      const double rl0 = __shfl_sync(0xffffffffu, rs, l0), rl1 = __shfl_sync(0xffffffffu, rs, l1);
+      A[(o + r) * kPanelLd + o + l0] = l0 < r ? a0 * rl0 : (l0 == r ? sd : 0.0);
+      A[(o + r) * kPanelLd + o + l1] = l1 < r ? a1 * rl1 : (l1 == r ? sd : 0.0);
+      Lp[r * 18 + l0] = l0 <= r ? e0 * rs : 0.0;
+      Lp[r * 18 + l1] = l1 <= r ? e1 * rs : 0.0;
+    }
+    __syncthreads();
+    // rows below the block, and b^T: columns j and 15 - j per thread
+    {
+      const int j = tid & 7, first = o + 16, total = nr + 1 - first;
+      const double* l0 = Lp + j * 18;
+      const double* l1 = Lp + (15 - j) * 18;
+      for (int i0 = 0; i0 < total; i0 += 4 * (kPanelThreads / 8)) {
+        double s0[4], s1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * (kPanelThreads / 8) + (tid >> 3);
+          s0[u] = s1[u] = 0.0;
+          if (i >= total) continue;
+          const double* ar = A + (first + i) * kPanelLd + o;
+          double acc = 0.0;
+#pragma unroll
+          for (int s = 0; s < 17; ++s) {
+            const bool lo = s <= j;
+            const int k = lo ? s : s - j - 1;
+            if (s == j + 1) {
+              s0[u] = acc;
+              acc = 0.0;
+            }
+            acc = fma(ar[k], lo ? l0[k] : l1[k], acc);
+          }
+          s1[u] = acc;
+        }
+        // a row's 16 values are read by the eight threads of its quarter warp only
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * (kPanelThreads / 8) + (tid >> 3);
+          if (i >= total) continue;
+          double* ar = A + (first + i) * kPanelLd + o;
+          ar[j] = s0[u];
+          ar[15 - j] = s1[u];
+        }
+      }
+    }
+    __syncthreads();
+    if (p + 1 < nblk) {
+      // columns to the right: the tile's lower 4 x 4 blocks, then the rows and b^T
+      const int m = 48 - o, nbk = m / 4, ntri = nbk * (nbk + 1) / 2 * 16, total = ntri + (rows + 1) * m;
+      const double* base = A + o;
+      for (int t = tid; t < total; t += kPanelThreads) {
+        int i, l;
+        if (t < ntri) {
+          const int blk = t >> 4;
+          int bi = (int)((sqrtf(8.0f * (float)blk + 1.0f) - 1.0f) * 0.5f);
+          while ((bi + 1) * (bi + 2) / 2 <= blk) ++bi;
+          while (bi * (bi + 1) / 2 > blk) --bi;
+          i = o + 16 + 4 * bi + ((t >> 2) & 3);
+          l = o + 16 + 4 * (blk - bi * (bi + 1) / 2) + (t & 3);
+        } else {
+          const int u = t - ntri;
+          i = 64 + u / m;
+          l = o + 16 + u % m;
+        }
+        const double* x = base + i * kPanelLd;
+        const double* y = base + l * kPanelLd;
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 16; k += 2) {
+          const double2 xv = *reinterpret_cast<const double2*>(x + k), yv = *reinterpret_cast<const double2*>(y + k);
+          s0 = fma(xv.x, yv.x, s0);
+          s1 = fma(xv.y, yv.y, s1);
+        }
+        A[i * kPanelLd + l] -= s0 + s1;
+      }
+      __syncthreads();
+    }
+  }
+  if (blockIdx.x == 0) {  // every CTA holds the same factor of the tile
+    double* Lo = Linv_all + (int64_t)kb * NB * NB;
+    for (int idx = tid; idx < 64 * 64; idx += kPanelThreads) {
+      const int r = idx >> 6, c = idx & 63, p = r >> 4;
+      double v = 0.0;
+      if (p != (c >> 4)) v = c < r ? A[r * kPanelLd + c] : 0.0;
+      else v = p < nblk ? Li[(p * 16 + (r & 15)) * 18 + (c & 15)] : (r == c ? 1.0 : 0.0);
+      Lo[idx] = v;
+    }
+    if (tid < 64) y[off + tid] = yb[tid];
+  }
+  // this CTA's rows of L, their digits and b_i -= L_i y
+  for (int idx = tid; idx < rows * 32; idx += kPanelThreads) {
+    const int r = idx >> 5, c = (idx & 31) * 2;
+    *reinterpret_cast<double2*>(S + (row0 + r) * ld + off + c) =
+        *reinterpret_cast<const double2*>(A + (64 + r) * kPanelLd + c);
+  }
+  for (int idx = tid; idx < rows * 8; idx += kPanelThreads) {
+    const int r = idx >> 3, k8 = idx & 7;
+    const int64_t i = row0 + r;
+    const double* x = A + (64 + r) * kPanelLd + 8 * k8;
+    // the row's exponent from its largest entry (its eight threads are a
+    // quarter warp); rows whose entries are not finite belong to a failed
+    // factorisation and take any value
+    double big = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) big = fmax(big, fabs(x[k]));
+    const unsigned mask = __activemask();
+#pragma unroll
+    for (int w = 1; w < 8; w <<= 1) big = fmax(big, __shfl_xor_sync(mask, big, w));
+    int xp = 0;
+    if (big > 0.0 && big < CUDART_INF) frexp(big, &xp);  // big < 2^xp
+    if (k8 == 0) ex[i] = -xp;
+    unsigned long long q[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double lim = 4611686018427387392.0;  // below 2^62
+      const double v = fmin(fmax(scalbn(x[k], 62 - xp), -lim), lim);
+      q[k] = ((unsigned long long)__double2ll_rn(v) + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+    }
+    // digit p of the tile of row i: rows of 128 bytes in 128-byte swizzle
+    __half* dst = digits + (i >> 6) * (kDigits * (int64_t)kDigitTile) + (i & 63) * 64 + ((k8 ^ (int)(i & 7)) * 8);
+    const __half2 bias = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));  // 1024 + 128
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // 1024 + byte has the bits 0x6400 | byte
+        const uint32_t u = 0x64006400u | (uint32_t)((q[2 * k] >> (56 - 8 * p)) & 0xff) |
+                           ((uint32_t)((q[2 * k + 1] >> (56 - 8 * p)) & 0xff) << 16);
+        const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&u), bias);
+        w[k] = *reinterpret_cast<const uint32_t*>(&v);
+      }
+      *reinterpret_cast<uint4*>(dst + p * kDigitTile) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  for (int r = tid >> 2; r < rows; r += kPanelThreads / 4) {  // rows is a multiple of 16: whole warps
+    const int q = tid & 3;
+    const double* x = A + (64 + r) * kPanelLd + q;
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 64; c += 4) s = fma(x[c], yb[q + c], s);
+    const unsigned mask = __activemask();
+    s += __shfl_xor_sync(mask, s, 1);
+    s += __shfl_xor_sync(mask, s, 2);
+    if (q == 0) b[row0 + r] -= s;
+  }
+}
+
+// Trailing update of panel kb on the tensor cores from the panel's digits:
+// S_IJ -= L_I L_J^T for the 64-column tiles J >= j0 and the row tiles I >= J,
+// one CTA per two row tiles and N of a tile's columns.  The eight sums of
+// digit products take N accumulator columns each; the operands arrive by bulk
+// copies with a barrier per digit, so that the MMAs start on the first.  The
+// epilogue makes each output's eight sums one FP64 number with integer
+// arithmetic and spends one FP64 instruction on it instead of 64.
+// N = 16 for the block column that the next panel waits for (four CTAs per
+// pair of tiles, a short epilogue: 11 us).  N = 32 for the bulk: its 160 KB of
+// operands leave room for a CTA of the next panel on the same SM, which runs
+// on the FP64 pipe meanwhile (with N = 64 and 192 KB the two take turns:
+// 4.2 ms against 3.2 ms for n = 2,388).
+// A bounded wait that runs out sets *flag = 6 (the step is then rejected).
+template <int N>
+struct SplitSmem {  // 1024-byte aligned (split_smem_bytes leaves room for it)
+  __half a[kDigits][2 * kDigitTile];
+  __half b[kDigits][N * 64];
+  uint64_t load_bar[kDigits], mma_bar;
+  uint32_t tmem_base, fail;
+  int32_t col_ex[N];
+};
+template <int N>
+constexpr size_t split_smem_bytes() { return sizeof(SplitSmem<N>) + 1024; }
+// v 2^e (rounded to nearest) without FP64 instructions; zero below the normal range.
+__device__ __forceinline__ double scaled_integer(long long v, int e) {
+  const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+  const int n = __clzll((long long)m);
+  const int ef = 1023 + 63 - n + e;  // exponent field
+  if (m == 0 || ef < 1) return 0.0;
+  // the rounded mantissa's leading one (and a carry out of it) adds to the field below it
+  const unsigned long long bits = ((unsigned long long)(ef - 1) << 52) + (((m << n) >> 11) + (((m << n) >> 10) & 1));
+  return __longlong_as_double((long long)(bits | ((unsigned long long)v & 0x8000000000000000ull)));
+}
+constexpr int kSplitThreads = 256;
+constexpr int kBulkN = 32;
+template <int N>
+__global__ void __maxnreg__(112) k_syrk_split(double* __restrict__ S, int64_t ld, int j0, int nb,
+                                                              const __half* __restrict__ digits,
+                                                              const int32_t* __restrict__ ex, int* __restrict__ flag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SplitSmem<N>& g = *reinterpret_cast<SplitSmem<N>*>(smem_raw + ((1024 - (umma::smem_addr(smem_raw) & 1023)) & 1023));
+  constexpr int kCols = 8 * N;    // accumulator columns
+  constexpr int C = N / 2;        // output columns per thread
+  constexpr int CH = C > 16 ? 16 : C;  // of which loaded at a time
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // CTA t: column tile jb = j0, j0 + 1, ... with ceil((nb - jb) / 2) pairs of row tiles each
+  int jb = j0, t = blockIdx.x / (64 / N);
+  const int cj = (blockIdx.x % (64 / N)) * N;  // first column inside the tile
+  while (t >= (nb - jb + 1) / 2) {
+    t -= (nb - jb + 1) / 2;
+    ++jb;
+  }
+  const int ib = jb + 2 * t;
+  const bool two = ib + 1 < nb;
+  if (tid == 0) {
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p) umma::mbar_init(&g.load_bar[p], 1);
+    umma::mbar_init(&g.mma_bar, 1);
+    g.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const __half* da = digits + ib * (kDigits * (int64_t)kDigitTile);
+    const __half* db = digits + jb * (kDigits * (int64_t)kDigitTile) + cj * 64;
+    constexpr uint32_t kBytes = kDigitTile * 2, kBytesB = N * 64 * 2;
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p) {
+      umma::mbar_expect(&g.load_bar[p], (two ? 2 * kBytes : kBytes) + kBytesB);
+      umma::bulk_load(g.a[p], da + p * kDigitTile, kBytes, &g.load_bar[p]);
+      if (two) umma::bulk_load(g.a[p] + kDigitTile, da + (kDigits + p) * (int64_t)kDigitTile, kBytes, &g.load_bar[p]);
+      umma::bulk_load(g.b[p], db + p * kDigitTile, kBytesB, &g.load_bar[p]);
+    }
+  }
+  if (tid >= 64 && tid < 64 + N) g.col_ex[tid - 64] = ex[(int64_t)jb * NB + cj + tid - 64];
+  if (warp == 0) {
+    __syncwarp();
+    umma::tmem_alloc(&g.tmem_base, kCols);
+    umma::tmem_relinquish();
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tm = g.tmem_base;
+  // this thread's outputs: a row of the pair of tiles, half of the columns
+  const int r = 32 * (warp & 3) + lane, c0 = C * (warp >> 2);
+  const bool mine = r < 64 || two;  // uniform over a warp
+  const int64_t row = (int64_t)ib * NB + r;
+  double* out = S + row * ld + (int64_t)jb * NB + cj + c0;
+  double x[CH];  // the first ones are loaded while the operands arrive
+  auto load = [&](int h) {
+#pragma unroll
+    for (int c = 0; c < CH; c += 2) {
+      const double2 w = *reinterpret_cast<const double2*>(out + h + c);
+      x[c] = w.x;
+      x[c + 1] = w.y;
+    }
+  };
+  int ei = 0;
+  if (mine) {
+    ei = ex[row];
+    load(0);
+  }
+  if (tid == 0) {
+    constexpr uint32_t idesc = umma::idesc_f16(128, N);
+    // descriptors advance by (bytes / 16)
+    const uint64_t da = umma::smem_desc_sw128(umma::smem_addr(g.a[0]));
+    const uint64_t db = umma::smem_desc_sw128(umma::smem_addr(g.b[0]));
+    constexpr uint32_t kStepA = sizeof(g.a[0]) / 16, kStepB = sizeof(g.b[0]) / 16;
+    bool ok = true;
+#pragma unroll
+    for (int s = 0; s < kDigits; ++s) {  // digit weights p + q = s: N accumulator columns each
+      ok = umma::mbar_wait(&g.load_bar[s], 0) && ok;
+      if (!ok) continue;
+#pragma unroll
+      for (int p = 0; p <= s; ++p)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma::mma_f16(tm + N * s, da + (p * kStepA + 2 * k), db + ((s - p) * kStepB + 2 * k), idesc, (p | k) != 0);
+    }
+    umma::mma_commit(&g.mma_bar);
+    if (!umma::mbar_wait(&g.mma_bar, 0) || !ok) g.fail = 1;
+  }
+  // one thread polls, the others wait at the barrier: 256 polling threads
+  // take the shared memory's bandwidth from the copies (16 us against 9)
+  __syncthreads();
+  const bool ok = g.fail == 0;
+  umma::fence_after_sync();
+  if (ok) {
+    if (mine) {
+      const uint32_t lanes = tm + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
+#pragma unroll 1
+      for (int h = 0; h < C; h += CH) {
+        if (h) load(h);
+#pragma unroll
+        for (int c8 = 0; c8 < CH; c8 += 8) {
+          uint32_t v[kDigits][8];
+#pragma unroll
+          for (int s = 0; s < kDigits; ++s) umma::tmem_ld8(lanes + N * s + h + c8, v[s]);
+          umma::tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            int d[kDigits];
+#pragma unroll
+            for (int s = 0; s < kDigits; ++s) d[s] = __float2int_rn(__uint_as_float(v[s][c]));
+            // sum_s d_s 2^(-12 - 8 s) in units of 2^-56, |sum| < 64
+            long long sum = 0;
+#pragma unroll
+            for (int s = 0; s < 6; ++s) sum = sum * 256 + d[s];
+            sum = sum * 16 + ((d[6] * 256 + d[7] + 2048) >> 12);
+            x[c8 + c] -= scaled_integer(sum, -56 - ei - g.col_ex[c0 + h + c8 + c]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < CH; c += 2) *reinterpret_cast<double2*>(out + h + c) = make_double2(x[c], x[c + 1]);
+      }
+    }
+  } else if (tid == 0) {
+    atomicExch(flag, 6);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  if (warp == 0) umma::tmem_dealloc(tm, kCols);
+}
+
+// Every tile's L^-1 (the backward substitution reads it) from k_panel64's
+// tiles, in place: the off-diagonal 16 x 16 blocks by increasing distance from
+// the diagonal, Li_IJ = -Li_II sum_{K=J..I-1} L_IK Li_KJ, one CTA per tile.
+// Off the panel chain, all tiles at once.
+__global__ void __launch_bounds__(256) k_tile_inverse(double* __restrict__ Linv_all) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* L = reinterpret_cast<double*>(smem_raw);  // [64][66]
+  double* Li = L + 64 * kPanelLd;                   // [64][66]
+  double* scr = Li + 64 * kPanelLd;                 // [3][16][16]
+  const int tid = threadIdx.x;
+  double* G = Linv_all + (int64_t)blockIdx.x * NB * NB;
+  for (int idx = tid; idx < 64 * 64; idx += 256) {
+    const int r = idx >> 6, c = idx & 63;
+    const double v = G[idx];
+    L[r * kPanelLd + c] = v;  // its diagonal blocks are not read
+    Li[r * kPanelLd + c] = (r >> 4) == (c >> 4) ? v : 0.0;
+  }
+  __syncthreads();
+  const int r = tid >> 4, c = tid & 15;
+#pragma unroll
+  for (int dist = 1; dist < 4; ++dist) {
+    // a thread's blocks and each block's 16-term pieces are independent chains
+    double sum[3][3];
+#pragma unroll
+    for (int J = 0; J < 4 - dist; ++J)
+#pragma unroll
+      for (int K = 0; K < dist; ++K) sum[J][K] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < 16; ++k)
+#pragma unroll
+      for (int J = 0; J < 4 - dist; ++J)
+#pragma unroll
+        for (int K = 0; K < dist; ++K)
+          sum[J][K] = fma(L[(16 * (J + dist) + r) * kPanelLd + 16 * (J + K) + k],
+                          Li[(16 * (J + K) + k) * kPanelLd + 16 * J + c], sum[J][K]);
+#pragma unroll
+    for (int J = 0; J < 4 - dist; ++J) {
+      double s = sum[J][0];
+#pragma unroll
+      for (int K = 1; K < dist; ++K) s += sum[J][K];
+      scr[J * 256 + tid] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int J = 0; J < 4 - dist; ++J) sum[J][0] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < 16; ++k)
+#pragma unroll
+      for (int J = 0; J < 4 - dist; ++J)
+        sum[J][0] = fma(Li[(16 * (J + dist) + r) * kPanelLd + 16 * (J + dist) + k], scr[J * 256 + k * 16 + c], sum[J][0]);
+#pragma unroll
+    for (int J = 0; J < 4 - dist; ++J) Li[(16 * (J + dist) + r) * kPanelLd + 16 * J + c] = -sum[J][0];
+    __syncthreads();
+  }
+  for (int idx = tid; idx < 64 * 64; idx += 256) G[idx] = Li[(idx >> 6) * kPanelLd + (idx & 63)];
+}
+constexpr size_t kTileInverseSmem = sizeof(double) * (2 * 64 * kPanelLd + 3 * 256);
+
+// Bytes of the FP64 factorisation's workspace: the digits of two panels (the
+// trailing update of a panel runs beside the next) with their rows' exponents, and y.
+size_t dense_cholesky_work_bytes(int64_t n_pad) {
+  return 2 * (size_t)(n_pad / NB) * kTileDigitBytes + (size_t)n_pad * (sizeof(double) + 2 * sizeof(int32_t));
+}
+
 // Opt the kernels into their dynamic shared memory (once per device and type;
 // called before any stream capture).
 template <typename T>
@@ -662,15 +1191,25 @@ void dense_cholesky_prepare() {
   static PerDeviceOnce once;
   once.run([] {
     const int sm = (int)dense_smem_bytes<T>();
-    GBBA_CUDA(cudaFuncSetAttribute(k_potrf_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)potrf_smem_bytes<T>()));
-    GBBA_CUDA(cudaFuncSetAttribute(k_trsm_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     GBBA_CUDA(cudaFuncSetAttribute(k_trsv_bwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    GBBA_CUDA(cudaFuncSetAttribute(k_syrk_wide<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)wide_smem_bytes<T>()));
-    if (std::is_same<T, float>::value)
+    if constexpr (std::is_same<T, float>::value) {
+      GBBA_CUDA(cudaFuncSetAttribute(k_potrf_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)potrf_smem_bytes<T>()));
+      GBBA_CUDA(cudaFuncSetAttribute(k_trsm_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+      GBBA_CUDA(cudaFuncSetAttribute(k_syrk_wide<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wide_smem_bytes<T>()));
       GBBA_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(umma::GemmSmem)));
+    } else {
+      GBBA_CUDA(cudaFuncSetAttribute(k_panel64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)panel64_smem(kPanelMaxRows)));
+      GBBA_CUDA(cudaFuncSetAttribute(k_syrk_split<kBulkN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)split_smem_bytes<kBulkN>()));
+      GBBA_CUDA(cudaFuncSetAttribute(k_syrk_split<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)split_smem_bytes<16>()));
+      GBBA_CUDA(cudaFuncSetAttribute(k_tile_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kTileInverseSmem));
+    }
   });
 }
 
@@ -715,7 +1254,7 @@ void launch_hi(gbba_handle* h, bool pdl, void (*k)(Exp...), unsigned grid, unsig
 // The side stream is joined back before the backward substitution, so the
 // sequence can be captured.
 // kTensor: the trailing update on the tensor cores (k_syrk_tc, FP32 only) or
-// on the FP32/FP64 pipes (k_syrk_wide).
+// on the FP32 pipes (k_syrk_wide).
 template <typename T, bool kTensor>
 void dense_cholesky_solve_impl(gbba_handle* h, T* S, int64_t n_pad, T* b, T* x, T* Linv_all, int* flag,
                                cudaStream_t st) {
@@ -758,10 +1297,64 @@ void dense_cholesky_solve_impl(gbba_handle* h, T* S, int64_t n_pad, T* b, T* x, 
               (const T*)Linv_all, b, x);
 }
 
+// FP64: the same look-ahead with the kernels above.  Per step k the call's
+// stream runs panel k, then panel k's update of block column k+1; the side
+// stream updates block columns k+2.. meanwhile.  The call's stream waits for
+// the side stream's step k-1 before step k's update (both write block column
+// k+1; the digits of panel k+1 then replace those of panel k-1).
+static void dense_cholesky_solve_fp64(gbba_handle* h, double* S, int64_t n, int64_t n_pad, double* b, double* x,
+                                      double* Linv_all, void* work, int* flag, cudaStream_t st) {
+  const int nb = (int)(n_pad / NB);
+  dense_cholesky_prepare<double>();
+  __half* digits[2];
+  digits[0] = static_cast<__half*>(work);
+  digits[1] = digits[0] + nb * kTileDigitBytes / 2;
+  double* y = reinterpret_cast<double*>(digits[1] + nb * kTileDigitBytes / 2);
+  int32_t* const exps[2] = {reinterpret_cast<int32_t*>(y + n_pad), reinterpret_cast<int32_t*>(y + n_pad) + n_pad};
+  bool side_pending = false;
+  for (int k = 0; k < nb; ++k) {
+    const int64_t below = (int64_t)(nb - k - 1) * NB;
+    // rows per CTA: 16, more when that would put two CTAs on an SM (they
+    // share its FP64 pipe, and each factors the diagonal tile)
+    const int R = (int)std::min<int64_t>(kPanelMaxRows, std::max<int64_t>(1, ceil_div(below, 16 * (int64_t)h->sm_count)) * 16);
+    const int nblk = k + 1 < nb ? 4 : (int)ceil_div(std::max<int64_t>(n - (int64_t)k * NB, 1), 16);
+    launch_hi(h, false, k_panel64, (unsigned)std::max<int64_t>(1, ceil_div(below, R)), kPanelThreads, panel64_smem(R),
+              st, S, n_pad, k, R, nblk, Linv_all, b, y, exps[k & 1], digits[k & 1], flag);
+    if (k + 1 == nb) break;
+    if (k + 2 < nb) {
+      GBBA_CUDA(cudaEventRecord(h->ev_main, st));
+      GBBA_CUDA(cudaStreamWaitEvent(h->side, h->ev_main, 0));
+    }
+    if (side_pending) GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
+    launch_hi(h, false, k_syrk_split<16>, (unsigned)((nb - k) / 2 * 4), kSplitThreads, split_smem_bytes<16>(), st, S, n_pad, k + 1,
+              nb, (const __half*)digits[k & 1], (const int32_t*)exps[k & 1], flag);
+    side_pending = k + 2 < nb;
+    if (side_pending) {
+      int64_t ctas = 0;
+      for (int j = k + 2; j < nb; ++j) ctas += (nb - j + 1) / 2;
+      k_syrk_split<kBulkN><<<(unsigned)(ctas * (64 / kBulkN)), kSplitThreads, split_smem_bytes<kBulkN>(), h->side>>>(S, n_pad, k + 2, nb, digits[k & 1],
+                                                                                  exps[k & 1], flag);
+      check_launch(h);
+      GBBA_CUDA(cudaEventRecord(h->ev_side, h->side));
+    }
+  }
+  if (side_pending) GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
+  k_tile_inverse<<<(unsigned)nb, 256, kTileInverseSmem, st>>>(Linv_all);
+  check_launch(h);
+  for (int kb = nb - 1; kb >= 0; --kb)
+    launch_hi(h, kb != nb - 1, k_trsv_bwd<double>, (unsigned)(kb + 1), 256, dense_smem_bytes<double>(), st,
+              (const double*)S, n_pad, kb, (const double*)Linv_all, y, x);
+}
+
+// n: unknowns of S (n_pad with the padding); work: dense_cholesky_work_bytes
+// (FP64 only).
 template <typename T>
-void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n_pad, T* b, T* x, T* Linv_all, int* flag, cudaStream_t st) {
-  if (std::is_same<T, float>::value && h->factor_tensor)
-    dense_cholesky_solve_impl<T, std::is_same<T, float>::value>(h, S, n_pad, b, x, Linv_all, flag, st);
+void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n, int64_t n_pad, T* b, T* x, T* Linv_all, void* work,
+                          int* flag, cudaStream_t st) {
+  if constexpr (std::is_same<T, double>::value)
+    dense_cholesky_solve_fp64(h, S, n, n_pad, b, x, Linv_all, work, flag, st);
+  else if (h->factor_tensor)
+    dense_cholesky_solve_impl<T, true>(h, S, n_pad, b, x, Linv_all, flag, st);
   else
     dense_cholesky_solve_impl<T, false>(h, S, n_pad, b, x, Linv_all, flag, st);
 }
@@ -772,7 +1365,9 @@ template void dense_cholesky_solve_impl<float, true>(gbba_handle*, float*, int64
                                                      cudaStream_t);
 template void dense_cholesky_prepare<double>();
 template void dense_cholesky_prepare<float>();
-template void dense_cholesky_solve<double>(gbba_handle*, double*, int64_t, double*, double*, double*, int*, cudaStream_t);
-template void dense_cholesky_solve<float>(gbba_handle*, float*, int64_t, float*, float*, float*, int*, cudaStream_t);
+template void dense_cholesky_solve<double>(gbba_handle*, double*, int64_t, int64_t, double*, double*, double*, void*,
+                                           int*, cudaStream_t);
+template void dense_cholesky_solve<float>(gbba_handle*, float*, int64_t, int64_t, float*, float*, float*, void*, int*,
+                                          cudaStream_t);
 
 }  // namespace gbba

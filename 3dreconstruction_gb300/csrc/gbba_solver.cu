@@ -42,7 +42,9 @@
 namespace gbba {
 
 template <typename T>
-void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n_pad, T* b, T* x, T* Linv_all, int* flag, cudaStream_t st);
+void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n, int64_t n_pad, T* b, T* x, T* Linv_all, void* work,
+                          int* flag, cudaStream_t st);
+size_t dense_cholesky_work_bytes(int64_t n_pad);
 template <typename T>
 void dense_cholesky_prepare();
 
@@ -2676,7 +2678,7 @@ struct Solve {
   unsigned long long* gmax_bits;
   unsigned long long* gmax_shards;  // gradient max norm of the fused linearisation (kGmaxShards slots)
   int *flag, *nonfinite;
-  void *S, *rhs, *zsol, *Linv, *Vinv, *gpv, *Wbuf, *What;
+  void *S, *rhs, *zsol, *Linv, *cwork, *Vinv, *gpv, *Wbuf, *What;
   double *part_mcc, *part_step_p, *part_step_c, *part_cost, *part_x, *scalars;
   int nb_obs, nb_pt, nb_cam, nb_x;
   // atomic-free Schur build (pair list in the handle's pair arena)
@@ -2776,6 +2778,7 @@ static void carve(A& a, Solve& s, size_t tsize) {
   s.rhs = a.template take<char>((size_t)s.n_pad * tsize);
   s.zsol = a.template take<char>((size_t)s.n_pad * tsize);
   s.Linv = a.template take<char>((size_t)n_s * kDenseTile * tsize);
+  s.cwork = a.template take<char>(tsize == 8 ? dense_cholesky_work_bytes(n_s) : 0);
   s.Vinv = a.template take<char>((size_t)s.np * 6 * tsize);
   s.gpv = a.template take<char>((size_t)s.np * 3 * tsize);
   s.part_mcc = a.template take<double>(s.nb_pt);
@@ -3554,7 +3557,7 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
         }
         break;
       case 2:
-        if (s.dense) dense_cholesky_solve<T>(h, S, s.n_pad, rhs, z, (T*)s.Linv, s.flag, st);
+        if (s.dense) dense_cholesky_solve<T>(h, S, s.n_red, s.n_pad, rhs, z, (T*)s.Linv, s.cwork, s.flag, st);
         else pcg_solve<M, T>(s, o, sum);
         break;
       case 3:

@@ -71,6 +71,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The same for K-major operands in 128-byte swizzle: rows of 128 bytes, eight
+// rows (1024 bytes, aligned) a swizzle atom, the 16-byte chunk c of row r at
+// chunk c ^ (r % 8), atoms 1024 bytes apart along M/N.  32 bytes of K on is
+// the start address + 32.  (Without the swizzle an MMA reads a 128-row operand
+// at 30 bytes a clock: 138 clocks for M = 128, K = 32 bytes, whatever N.)
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
 // Instruction descriptor of kind::tf32: FP32 accumulator (bits 4-5 = 1),
 // A and B TF32 (bits 7-9, 10-12 = 2), both K-major (bits 15, 16 = 0),
 // N / 8 at bits 17-22, M / 16 at bits 24-28.
@@ -87,6 +96,34 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// Instruction descriptor of kind::f16 with FP16 operands: FP32 accumulator
+// (bits 4-5 = 1), A and B FP16 (bits 7-9, 10-12 = 0), both K-major, N / 8 at
+// bits 17-22, M / 16 at bits 24-28.
+__host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// D (+)= A B^T with FP16 operands (K = 16 per instruction), issued by a single thread.
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// An mbarrier's arrival that also announces `bytes` of asynchronous copies.
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// Asynchronous copy of `bytes` contiguous bytes (16-byte aligned, a multiple
+// of 16) into shared memory, counted on the mbarrier.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_addr(dst)),
+               "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
 }
 // The mbarrier receives one arrival once every MMA this thread issued before
 // has completed.
@@ -113,6 +150,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
+
+// 8 consecutive accumulator columns of this thread's tensor-memory lane; the
+// values are valid after tmem_ld_wait.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t r[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ float tf32_round(float x) {
   uint32_t r;
