@@ -11,17 +11,14 @@
 // 64x64 tile is full and no kernel needs bounds checks.
 //
 // Algorithm (right-looking, block size 64, one launch sequence per panel k):
-//   potrf_diag : factor S_kk = L_kk L_kk^T in shared memory, form L_kk^-1,
-//                and finish the forward substitution of block k: y_k = L_kk^-1 b_k
-//   trsm_panel : L_ik = S_ik L_kk^-T for every i > k, and b_i -= L_ik y_k
-//                (forward substitution fused into the panel solve)
-//   syrk       : S_ij -= L_ik L_jk^T for k < j <= i (trailing update)
+//   panel : S_kk = L_kk L_kk^T (by every CTA), y_k = L_kk^-1 b_k,
+//           L_ik = S_ik L_kk^-T and b_i -= L_ik y_k for i > k
+//   syrk  : S_ij -= L_ik L_jk^T for k < j <= i (trailing update)
 // then the backward substitution L^T x = y, right-looking by block rows:
 //   trsv_bwd(k): x_k = L_kk^-T y_k; y_j -= L_kj^T x_k for j < k.
 // A non-positive pivot sets *flag (LINEAR_SOLVER_FAILURE in ceres terms).
-// That is the FP32 path; the FP64 path has its own kernels for the panel and
-// the trailing update (k_panel64, k_syrk_split) and shares the backward
-// substitution.
+// FP32: k_panel32 and k_syrk_tc or k_syrk_wide; FP64: k_panel64 and
+// k_syrk_split; both: k_trsv_bwd.
 #include <cuda_fp16.h>
 #include <math_constants.h>
 
@@ -35,7 +32,7 @@ namespace gbba {
 constexpr int NB = 64;
 
 // Two padded 64x64 tiles (plus a few vectors) live in dynamic shared memory:
-// 66.5 KB in FP64, above the 48 KB static limit.
+// 66.5 KB in FP64, above the 48 KB static limit (the backward substitution).
 template <typename T>
 __device__ __forceinline__ T (*tile_at(int i))[NB + 1] {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -48,29 +45,6 @@ __device__ __forceinline__ T* vec_at(int i) {
 }
 template <typename T>
 constexpr size_t dense_smem_bytes() { return (size_t)2 * NB * (NB + 1) * sizeof(T) + 2 * NB * sizeof(T); }
-
-// Copy the contiguous 64x64 tile at src (row stride 64) with L2-only loads
-// (ld.global.cg): for data written by a kernel that may still have been
-// running when this kernel started (programmatic dependent launch), so that
-// no line cached in L1 before that kernel finished can be read.
-template <typename T>
-__device__ __forceinline__ void load_tile_cg(T (*dst)[NB + 1], const T* src, int tid) {
-  using V = typename Vec16<T>::type;
-  constexpr int W = Vec16<T>::n, PER_ROW = NB / W, ITER = NB * PER_ROW / 256;
-  V v[ITER];
-#pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int idx = tid + it * 256, r = idx / PER_ROW, c = (idx % PER_ROW) * W;
-    v[it] = __ldcg(reinterpret_cast<const V*>(src + r * NB + c));
-  }
-#pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int idx = tid + it * 256, r = idx / PER_ROW, c = (idx % PER_ROW) * W;
-    const T* e = reinterpret_cast<const T*>(&v[it]);
-#pragma unroll
-    for (int w = 0; w < W; ++w) dst[r][c + w] = e[w];
-  }
-}
 
 // Copy the 64x64 tile at src (row stride ld) into a padded shared tile.  All
 // of a thread's global loads are issued before its shared stores so that
@@ -100,369 +74,350 @@ __device__ __forceinline__ void load_tile(T (*dst)[NB + 1], const T* __restrict_
 // decided on the FP64 cost.
 __device__ __forceinline__ float pivot_rcp(float d) { return __fdividef(1.0f, d); }
 
-// Factor the diagonal tile: S_kk = L L^T (written back into S's lower
-// triangle, zeros above), L^-1 (into Linv_all), and y_k = L^-1 b_k.
+// Panel kb (FP32): the diagonal tile's factor and inverse, and one 64 x 64
+// tile of the block column below it per CTA:
+//   (with upd) S_kk -= P P^T and S_ib,kb -= L_ib,kb-1 P^T, P = L_kb,kb-1 (the
+//              previous panel's update of this block column)
+//   S_kk = L_kk L_kk^T, y_kb = L_kk^-1 b_kb,
+//   L_ib,kb = S_ib,kb L_kk^-T,  b_ib -= L_ib,kb y_kb
+//   (with ops) the tile's TF32 operands of the trailing update (k_syrk_tc).
+// Every CTA factors the diagonal tile itself: that costs no time (the chain of
+// pivots bounds it) and saves a kernel and its hand-over per panel.  S_kk and
+// b_kb stay as they are (other CTAs may still have to read them): L_kk^-1 goes
+// to Linv, y_kb to y.  A grid of one CTA without a tile serves the last panel.
 //
-// Blocked right-looking factorisation of the 64 x 64 tile in shared memory
-// over four 16-column panels p (offset o = 16p):
-//   1. warp 0 factors the 16 x 16 diagonal block: outer-product LDL^T with
-//      the same row operations applied to an identity block E (so that
-//      E = L_u^-1 at the end); lane (r, h) holds row r, columns 8h..8h+7 of
-//      both in registers, pivots are broadcast through shared memory with
-//      only __syncwarp between steps;
-//   2. panel solve  L_ip = A_ip L_pp^-T  for the rows below (all threads);
-//   3. trailing update  A_il -= L_ip L_lp^T  inside the tile (all threads);
-// then the off-diagonal 16 x 16 blocks of L^-1 by increasing distance from
-// the diagonal,  Li_IJ = -Li_II sum_{K=J..I-1} L_IK Li_KJ,  and y = L^-1 b.
+// Warps 0..7 factor the tile in shared memory, four 16-column panels p
+// (offset o = 16p):
+//   1. warps 0..3: the 16 x 16 diagonal block, outer-product LDL^T with the
+//      same row operations applied to an identity block (its inverse).  Of
+//      the 16 columns l at pivot j, those right of j take the elimination of
+//      the block, the others that of the identity (its row j ends at column
+//      j); warp w holds columns w, w + 4, w + 8, w + 12 of all rows and a
+//      pivot's column is passed on through shared memory, one barrier of the
+//      four warps per pivot;
+//   2. panel solve  L_ip = A_ip L_pp^-T  for the rows below;
+//   3. trailing update  A_il -= L_ip L_lp^T  inside the tile.
+// Warps 8..15 apply the previous panel's update to the CTA's own tile first,
+// then form row p of 16 x 16 blocks of L^-1 as soon as diagonal block p is
+// factored, Li_pJ = -Li_pp sum_{K=J..p-1} L_pK Li_KJ, beside steps 2, 3 and the
+// next block's pivots.  All warps then multiply by L_kk^-T.
 // A non-positive (or non-finite) pivot is replaced by 1 and sets *flag.
-constexpr int kPotrfThreads = 256;
+// Medium workload (94 panels): 22 us a panel, against 25 + 10 us for a
+// diagonal kernel (one warp per block, pivots by shuffles) and a panel kernel.
+constexpr int kPanel32Threads = 512;
 constexpr int kTileLd = NB + 4;  // 16-byte aligned rows
-template <typename T>
-constexpr size_t potrf_smem_bytes() {
-  return sizeof(T) * ((size_t)2 * NB * kTileLd   // A / L, L^-1
-                      + 3 * 16 * 16              // scratch of the inverse blocks
-                      + 4 * 16 + 4               // warp-0 broadcast buffers
-                      + 2 * NB);                 // b, pivots
+constexpr int kTileF = NB * kTileLd;
+constexpr size_t kPanel32Smem = sizeof(float) * (5 * (size_t)kTileF + 3 * 256 + 256 + 2 * NB);
+// Operands of the TF32 trailing update, per 64 x 64 tile: [hi, lo][32 columns]
+// of 64 rows x 128 bytes in 128-byte swizzle.
+constexpr int kOpsPiece = 64 * 32;
+constexpr int kOpsTile = 4 * kOpsPiece;
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPotrfThreads) k_potrf_diag(T* __restrict__ S, int64_t ld, int kb,
-                                                              T* __restrict__ Linv_all, T* __restrict__ b,
-                                                              int* __restrict__ flag, int upd) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);  // [64][kTileLd]: A, overwritten by L
-  T* Li = A + NB * kTileLd;               // [64][kTileLd]: L^-1
-  T* scr = Li + NB * kTileLd;             // [3][16][16]
-  T* bc = scr + 3 * 256;                  // [2][16] pivot column
-  T* br = bc + 32;                        // [2][16] row of E
-  T* rp = br + 32;                        // [2] 1/d (+2 padding)
-  T* yb = rp + 4;                         // [64]
-  T* dv = yb + NB;                        // [64] pivots of the current panel
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t off = (int64_t)kb * NB;
-  // the panel solve of this block column may start now: it reads L^-1 and y
-  // only after griddepcontrol.wait, i.e. after this kernel has completed
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // load the tile (lower part is what is used) and b; with upd, also the
-  // previous panel's block P = L_{kb,kb-1} (staged in the L^-1 buffer)
-#pragma unroll
-  for (int it = 0; it < NB * NB / 4 / kPotrfThreads; ++it) {
-    const int idx = tid + it * kPotrfThreads, r = idx >> 4, c = (idx & 15) * 4;
-    T v[4];
-    ld4<T>(S + (off + r) * ld + off + c, v);
-    st4<T>(A + r * kTileLd + c, v);
-    if (upd) {
-      ld4<T>(S + (off + r) * ld + off - NB + c, v);
-      st4<T>(Li + r * kTileLd + c, v);
-    }
-  }
-  if (tid < NB) yb[tid] = b[off + tid];
-  __syncthreads();
-  if (upd) {
-    // A -= P P^T (thread: rows 4(tid>>4).., columns 4(tid&15)..)
-    const int r0 = 4 * (tid >> 4), l0 = 4 * (tid & 15);
-    T acc[4][4] = {};
+// acc(4 x 4) += X Y^T over 64 columns, rows ty + 16 i of X and tx + 16 j of Y
+// (tiles of row stride kTileLd: a quarter warp's 16-byte loads touch all banks).
+__device__ __forceinline__ void tile_xyt(const float* X, const float* Y, int ty, int tx, float acc[4][4]) {
 #pragma unroll 4
-    for (int k4 = 0; k4 < NB; k4 += 4) {
-      T xi[4][4], xl[4][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        ld4<T>(Li + (r0 + q) * kTileLd + k4, xi[q]);
-        ld4<T>(Li + (l0 + q) * kTileLd + k4, xl[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int w = 0; w < 4; ++w)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[q][w] += xi[q][k] * xl[w][k];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      T v[4];
-      ld4<T>(A + (r0 + q) * kTileLd + l0, v);
-#pragma unroll
-      for (int w = 0; w < 4; ++w) v[w] -= acc[q][w];
-      st4<T>(A + (r0 + q) * kTileLd + l0, v);
-    }
-    __syncthreads();
-  }
-  // clear L^-1
-#pragma unroll
-  for (int it = 0; it < NB * NB / 4 / kPotrfThreads; ++it) {
-    const int idx = tid + it * kPotrfThreads, r = idx >> 4, c = (idx & 15) * 4;
-    const T z[4] = {T(0), T(0), T(0), T(0)};
-    st4<T>(Li + r * kTileLd + c, z);
-  }
-  __syncthreads();
-
-  for (int p = 0; p < 4; ++p) {
-    const int o = 16 * p;
-    // ---- 1. diagonal 16 x 16 block, warp 0
-    if (warp == 0) {
-      const int r = lane & 15, h = lane >> 4;
-      T a[8], e[8];
-      ld4<T>(A + (o + r) * kTileLd + o + 8 * h, a);
-      ld4<T>(A + (o + r) * kTileLd + o + 8 * h + 4, a + 4);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) e[q] = (r == 8 * h + q) ? T(1) : T(0);
-      // pivot j: lane (i, h') holds a_ij in a[j & 7] when h' = j >> 3, and
-      // row j of E lives in lanes (j, 0) and (j, 1); everything a lane needs
-      // is fetched with independent shuffles (no shared-memory round trip)
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int hs = 16 * (j >> 3);  // lane offset of the owners of column j
-        T d = __shfl_sync(0xffffffffu, a[j & 7], j + hs);
-        const T cr = __shfl_sync(0xffffffffu, a[j & 7], r + hs);
-        T cl[8], rl[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          cl[q] = __shfl_sync(0xffffffffu, a[j & 7], 8 * h + q + hs);
-          rl[q] = __shfl_sync(0xffffffffu, e[q], j + 16 * h);
-        }
-        if (!(d > T(0) && d - d == T(0))) {  // non-positive, NaN or infinite pivot
-          d = T(1);
-          if (lane == 0) atomicExch(flag, 1);
-        }
-        if (lane == 0) dv[o + j] = d;
-        const T m = (r > j) ? cr * pivot_rcp(d) : T(0);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const T c = (8 * h + q > j) ? cl[q] : T(0);
-          a[q] -= m * c;
-          e[q] -= m * rl[q];
-        }
-      }
-      __syncwarp();
-      // L_pp = L_u D^1/2, L_pp^-1 = D^-1/2 E: sqrt(d) and 1/sqrt(d) once per
-      // pivot (lanes 0..15 in parallel), then products only
-      T* sqd = bc;       // [16] sqrt(d), reusing the broadcast buffers
-      T* rsd = bc + 16;  // [16] 1/sqrt(d)
-      if (lane < 16) {
-        const T sd = sqrt(dv[o + lane]);
-        sqd[lane] = sd;
-        rsd[lane] = T(1) / sd;
-      }
-      __syncwarp();
-      const T rr = rsd[r];
-      T rl8[8];
-      ld4<T>(rsd + 8 * h, rl8);
-      ld4<T>(rsd + 8 * h + 4, rl8 + 4);
-      T lv[8], iv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int l = 8 * h + q;
-        lv[q] = (l < r) ? a[q] * rl8[q] : (l == r ? sqd[r] : T(0));
-        iv[q] = (l <= r) ? e[q] * rr : T(0);
-      }
-      st4<T>(A + (o + r) * kTileLd + o + 8 * h, lv);
-      st4<T>(A + (o + r) * kTileLd + o + 8 * h + 4, lv + 4);
-      st4<T>(Li + (o + r) * kTileLd + o + 8 * h, iv);
-      st4<T>(Li + (o + r) * kTileLd + o + 8 * h + 4, iv + 4);
-    }
-    __syncthreads();
-    if (p == 3) break;
-    // ---- 2. panel solve: rows o+16..63, L_ic = sum_k A_ik Li_pp[c][k]
-    const int rows = NB - o - 16;
-    T pv[3];
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int idx = tid + u * kPotrfThreads;
-      pv[u] = T(0);
-      if (idx < rows * 16) {
-        const int i = o + 16 + (idx >> 4), c = idx & 15;
-        T s4[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-        for (int k4 = 0; k4 < 16; k4 += 4) {
-          T av[4], lv[4];
-          ld4<T>(A + i * kTileLd + o + k4, av);
-          ld4<T>(Li + (o + c) * kTileLd + o + k4, lv);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) s4[k] += av[k] * lv[k];
-        }
-        pv[u] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int idx = tid + u * kPotrfThreads;
-      if (idx < rows * 16) A[(o + 16 + (idx >> 4)) * kTileLd + o + (idx & 15)] = pv[u];
-    }
-    __syncthreads();
-    // ---- 3. trailing update inside the tile: 4 x 4 output blocks, lower blocks only
-    {
-      const int nbk = rows / 4;  // 4-row blocks of the trailing part
-      for (int t = tid; t < nbk * nbk; t += kPotrfThreads) {
-        const int bi = t / nbk, bl = t % nbk;
-        if (bl > bi) continue;
-        const int i0 = o + 16 + 4 * bi, l0 = o + 16 + 4 * bl;
-        T acc[4][4] = {};
-#pragma unroll
-        for (int k4 = 0; k4 < 16; k4 += 4) {
-          T xi[4][4], xl[4][4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            ld4<T>(A + (i0 + q) * kTileLd + o + k4, xi[q]);
-            ld4<T>(A + (l0 + q) * kTileLd + o + k4, xl[q]);
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int w = 0; w < 4; ++w)
-#pragma unroll
-              for (int k = 0; k < 4; ++k) acc[q][w] += xi[q][k] * xl[w][k];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          T v[4];
-          ld4<T>(A + (i0 + q) * kTileLd + l0, v);
-#pragma unroll
-          for (int w = 0; w < 4; ++w) v[w] -= acc[q][w];
-          st4<T>(A + (i0 + q) * kTileLd + l0, v);
-        }
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- off-diagonal blocks of L^-1, by distance from the diagonal
-  for (int dist = 1; dist < 4; ++dist) {
-    const int nblk = 4 - dist;  // blocks (J + dist, J), J = 0..nblk-1
-    // T_IJ = sum_{K=J}^{I-1} L_IK Li_KJ
-    for (int idx = tid; idx < nblk * 256; idx += kPotrfThreads) {
-      const int J = idx >> 8, I = J + dist, r = (idx >> 4) & 15, c = idx & 15;
-      T s4[4] = {T(0), T(0), T(0), T(0)};
-      for (int K = J; K < I; ++K) {
-        const T* ar = A + (16 * I + r) * kTileLd + 16 * K;
-#pragma unroll
-        for (int k4 = 0; k4 < 16; k4 += 4) {
-          T av[4];
-          ld4<T>(ar + k4, av);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) s4[k] += av[k] * Li[(16 * K + k4 + k) * kTileLd + 16 * J + c];
-        }
-      }
-      scr[idx] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-    }
-    __syncthreads();
-    // Li_IJ = -Li_II T_IJ
-    for (int idx = tid; idx < nblk * 256; idx += kPotrfThreads) {
-      const int J = idx >> 8, I = J + dist, r = (idx >> 4) & 15, c = idx & 15;
-      T s4[4] = {T(0), T(0), T(0), T(0)};
-      const T* lr = Li + (16 * I + r) * kTileLd + 16 * I;
-#pragma unroll
-      for (int k4 = 0; k4 < 16; k4 += 4) {
-        T lv[4];
-        ld4<T>(lr + k4, lv);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s4[k] += lv[k] * scr[(J << 8) + (k4 + k) * 16 + c];
-      }
-      Li[(16 * I + r) * kTileLd + 16 * J + c] = -((s4[0] + s4[1]) + (s4[2] + s4[3]));
-    }
-    __syncthreads();
-  }
-
-  // ---- y = L^-1 b (4 threads per row), then write L and L^-1
-  {
-    const int r = tid >> 2, q = tid & 3;
-    T s = T(0);
-#pragma unroll
-    for (int c = 0; c < 16; ++c) s += Li[r * kTileLd + 16 * q + c] * yb[16 * q + c];
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (q == 0) b[off + r] = s;
-  }
-#pragma unroll
-  for (int it = 0; it < NB * NB / 4 / kPotrfThreads; ++it) {
-    const int idx = tid + it * kPotrfThreads, r = idx >> 4, c = (idx & 15) * 4;
-    T v[4], w[4];
-    ld4<T>(A + r * kTileLd + c, v);
-    ld4<T>(Li + r * kTileLd + c, w);
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (c + e > r) v[e] = T(0);
-    st4<T>(S + (off + r) * ld + off + c, v);
-    st4<T>(Linv_all + (int64_t)kb * NB * NB + r * NB + c, w);
-  }
-}
-
-// 64x64 tile product helper: acc(4x4 per thread) += X[rows] . Y[cols]^T over l.
-template <typename T>
-__device__ __forceinline__ void tile_xyt(const T (*X)[NB + 1], const T (*Y)[NB + 1], int ty, int tx, T acc[4][4]) {
-#pragma unroll 8
-  for (int l = 0; l < NB; ++l) {
-    T xr[4], yc[4];
+  for (int k4 = 0; k4 < NB; k4 += 4) {
+    float x[4][4], y[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      xr[i] = X[ty * 4 + i][l];
-      yc[i] = Y[tx * 4 + i][l];
+      ld4<float>(X + (ty + 16 * i) * kTileLd + k4, x[i]);
+      ld4<float>(Y + (tx + 16 * i) * kTileLd + k4, y[i]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += xr[i] * yc[j];
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[i][j] += x[i][k] * y[j][k];
+  }
+}
+// One or two 64 x 64 tiles (row stride ld) into shared memory by 256 threads,
+// all loads in flight at once.
+__device__ __forceinline__ void load_tiles32(float* d0, const float* __restrict__ s0, float* d1,
+                                             const float* __restrict__ s1, int64_t ld, int t) {
+  float v[2][4][4];
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int64_t at = ((t + it * 256) >> 4) * ld + (t & 15) * 4;
+    ld4<float>(s0 + at, v[0][it]);
+    if (s1) ld4<float>(s1 + at, v[1][it]);
+  }
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int at = ((t + it * 256) >> 4) * kTileLd + (t & 15) * 4;
+    st4<float>(d0 + at, v[0][it]);
+    if (s1) st4<float>(d1 + at, v[1][it]);
   }
 }
 
-// Panel solve of block column kb: for tile ib = kb + 1 + blockIdx.x,
-//   (with upd) S_ib,kb -= L_ib,kb-1 L_kb,kb-1^T   (the previous panel's
-//                                                  update of this tile)
-//   L_ib,kb = S_ib,kb L_kb,kb^-T,   b_ib -= L_ib,kb y_kb
-// (the forward substitution is fused into the panel solve).
-template <typename T>
-__global__ void __launch_bounds__(256) k_trsm_panel(T* __restrict__ S, int64_t ld, int kb, const T* Linv_all, T* b,
-                                                    int upd) {
-  T(*A)[NB + 1] = tile_at<T>(0);
-  T(*Li)[NB + 1] = tile_at<T>(1);
-  T* y = vec_at<T>(0);
-  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
+__global__ void __launch_bounds__(kPanel32Threads) k_panel32(float* __restrict__ S, int64_t ld, int kb, int nb,
+                                                             float* __restrict__ Linv_all, float* __restrict__ b,
+                                                             float* __restrict__ y, float* __restrict__ ops,
+                                                             int* __restrict__ flag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* A = reinterpret_cast<float*>(smem_raw);  // [64][kTileLd]: S_kk, overwritten by L_kk
+  float* Li = A + kTileF;                         // [64][kTileLd]: L_kk^-1
+  float* P = Li + kTileF;                         // [64][kTileLd]: L_kb,kb-1
+  float* T1 = P + kTileF;                         // [64][kTileLd]: L_ib,kb-1, then L_ib,kb
+  float* T2 = T1 + kTileF;                        // [64][kTileLd]: S_ib,kb
+  float* scr = T2 + kTileF;                       // [3][16][16] products of the inverse blocks
+  float* cb = scr + 3 * 256;                      // [16][16] the pivots' columns
+  float* yb = cb + 256;                           // [64] b_kb
+  float* yv = yb + NB;                            // [64] y_kb
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t off = (int64_t)kb * NB;
   const int64_t ib = kb + 1 + blockIdx.x;
-  const int64_t r0 = ib * NB, c0 = (int64_t)kb * NB;
-  T a[4][4];
+  const bool has_tile = ib < nb;
+  const bool upd = kb > 0;
+  const int64_t r0 = ib * NB;
+  // barriers; one of its own per diagonal block (an arrival must not run ahead
+  // into a phase that the other side has not entered)
+  enum { kBarA = 1, kBarDiag = 2, kBarB = 3, kBarStage = 4 /* .. 7 */ };
+  if (tid < 256) {
+    load_tiles32(A, S + off * ld + off, P, upd ? S + off * ld + off - NB : nullptr, ld, tid);
+    if (tid < NB) yb[tid] = b[off + tid];
+    if (upd) {
+      __syncthreads();  // P is read by all
+      const int ty = tid >> 4, tx = tid & 15;
+      float acc[4][4] = {};
+      tile_xyt(P, P, ty, tx, acc);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) ld4<T>(S + (r0 + ty * 4 + i) * ld + c0 + tx * 4, a[i]);
-  if (upd) {
-    load_tile<T>(A, S + r0 * ld + c0 - NB, ld, tid);
-    load_tile<T>(Li, S + c0 * ld + c0 - NB, ld, tid);
-    __syncthreads();
-    T acc[4][4] = {};
-    tile_xyt<T>(A, Li, ty, tx, acc);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j) A[(ty + 16 * i) * kTileLd + tx + 16 * j] -= acc[i][j];
+    }
+    bar_sync(kBarA, 256);
+    for (int p = 0; p < 4; ++p) {
+      const int o = 16 * p;
+      // ---- 1. diagonal 16 x 16 block
+      if (warp < 4) {
+        const int r = lane & 15;
+        const int l0 = warp + 4 * (lane >> 4), l1 = l0 + 8;  // this lane's columns of row r
+        float a0 = A[(o + r) * kTileLd + o + l0], a1 = A[(o + r) * kTileLd + o + l1];
+        float e0 = r == l0 ? 1.f : 0.f, e1 = r == l1 ? 1.f : 0.f;
+        if (l0 == 0) cb[r] = a0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) a[i][j] -= acc[i][j];
-    __syncthreads();
+        for (int j = 0; j < 16; ++j) {
+          bar_sync(kBarDiag, 128);
+          const float* col = cb + 16 * j;
+          float d = col[j];
+          const float cr = col[r], c0 = col[l0], c1 = col[l1];
+          const float f0 = __shfl_sync(0xffffffffu, e0, j + (lane & 16)), f1 = __shfl_sync(0xffffffffu, e1, j + (lane & 16));
+          if (!(d > 0.f && d - d == 0.f)) {  // non-positive, NaN or infinite pivot
+            d = 1.f;
+            if (tid == 0) {
+              cb[17 * j] = 1.f;
+              atomicExch(flag, 1);
+            }
+          }
+          const float m = r > j ? cr * pivot_rcp(d) : 0.f;
+          auto column = [&](int l, float& av, float& ev, float cl, float fl) {
+            const bool right = l > j;
+            const float v = fmaf(-m, right ? cl : fl, right ? av : ev);
+            av = right ? v : av;
+            ev = right ? ev : v;
+            if (l == j + 1) cb[16 * (j + 1) + r] = av;
+          };
+          if (j + 1 < 8) {  // the next pivot's column first
+            column(l0, a0, e0, c0, f0);
+            column(l1, a1, e1, c1, f1);
+          } else {
+            column(l1, a1, e1, c1, f1);
+            column(l0, a0, e0, c0, f0);
+          }
+        }
+        bar_sync(kBarDiag, 128);
+        // L_pp = L_u D^1/2, L_pp^-1 = D^-1/2 L_u^-1
+        const float sd = sqrtf(cb[17 * r]), rs = 1.f / sd;
+        const float rl0 = __shfl_sync(0xffffffffu, rs, l0), rl1 = __shfl_sync(0xffffffffu, rs, l1);
+        A[(o + r) * kTileLd + o + l0] = l0 < r ? a0 * rl0 : (l0 == r ? sd : 0.f);
+        A[(o + r) * kTileLd + o + l1] = l1 < r ? a1 * rl1 : (l1 == r ? sd : 0.f);
+        Li[(o + r) * kTileLd + o + l0] = l0 <= r ? e0 * rs : 0.f;
+        Li[(o + r) * kTileLd + o + l1] = l1 <= r ? e1 * rs : 0.f;
+      }
+      bar_sync(kBarA, 256);
+      bar_arrive(kBarStage + p, kPanel32Threads);  // warps 8..15 take row p of L^-1
+      if (p == 3) break;
+      // ---- 2. panel solve: rows o+16..63, L_ic = sum_k A_ik Li_pp[c][k]
+      const int rows = NB - o - 16;
+      float pv[3];
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int idx = tid + u * 256;
+        pv[u] = 0.f;
+        if (idx < rows * 16) {
+          const int i = o + 16 + (idx >> 4), c = idx & 15;
+          float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int k4 = 0; k4 < 16; k4 += 4) {
+            float av[4], lv[4];
+            ld4<float>(A + i * kTileLd + o + k4, av);
+            ld4<float>(Li + (o + c) * kTileLd + o + k4, lv);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s4[k] += av[k] * lv[k];
+          }
+          pv[u] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        }
+      }
+      __syncwarp();  // a row's 16 values are read by its half warp only
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int idx = tid + u * 256;
+        if (idx < rows * 16) A[(o + 16 + (idx >> 4)) * kTileLd + o + (idx & 15)] = pv[u];
+      }
+      bar_sync(kBarA, 256);
+      // ---- 3. trailing update inside the tile, a lower 16 x 16 block at a time
+      {
+        const int r = tid >> 4, c = tid & 15;
+#pragma unroll
+        for (int I = 1; I < 4; ++I)
+#pragma unroll
+          for (int J = 1; J <= I; ++J) {
+            if (J <= p || I <= p) continue;
+            const float* x = A + (16 * I + r) * kTileLd + o;
+            const float* z = A + (16 * J + c) * kTileLd + o;
+            float acc = 0.f;
+#pragma unroll
+            for (int k4 = 0; k4 < 16; k4 += 4) {
+              float xv[4], zv[4];
+              ld4<float>(x + k4, xv);
+              ld4<float>(z + k4, zv);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) acc += xv[k] * zv[k];
+            }
+            A[(16 * I + r) * kTileLd + 16 * J + c] -= acc;
+          }
+      }
+      bar_sync(kBarA, 256);
+    }
+  } else {
+    const int t = tid - 256, ty = t >> 4, tx = t & 15;
+    if (has_tile) load_tiles32(T2, S + r0 * ld + off, T1, upd ? S + r0 * ld + off - NB : nullptr, ld, t);
+    if (upd) {
+      __syncthreads();
+      if (has_tile) {
+        float acc[4][4] = {};
+        tile_xyt(T1, P, ty, tx, acc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) T2[(ty + 16 * i) * kTileLd + tx + 16 * j] -= acc[i][j];
+      }
+    }
+    // the blocks of L^-1 above the diagonal
+    for (int idx = t; idx < NB * NB; idx += 256)
+      if ((idx & 63) >> 4 > idx >> 10) Li[(idx >> 6) * kTileLd + (idx & 63)] = 0.f;
+    for (int I = 0; I < 4; ++I) {
+      bar_sync(kBarStage + I, kPanel32Threads);
+      // T_IJ = sum_{K=J}^{I-1} L_IK Li_KJ, then Li_IJ = -Li_II T_IJ
+      for (int J = 0; J < I; ++J) {
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int K = J; K < I; ++K) {
+          const float* ar = A + (16 * I + ty) * kTileLd + 16 * K;
+#pragma unroll
+          for (int k4 = 0; k4 < 16; k4 += 4) {
+            float av[4];
+            ld4<float>(ar + k4, av);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s4[k] += av[k] * Li[(16 * K + k4 + k) * kTileLd + 16 * J + tx];
+          }
+        }
+        scr[(J << 8) + t] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      }
+      bar_sync(kBarB, 256);
+      for (int J = 0; J < I; ++J) {
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+        const float* lr = Li + (16 * I + ty) * kTileLd + 16 * I;
+#pragma unroll
+        for (int k4 = 0; k4 < 16; k4 += 4) {
+          float lv[4];
+          ld4<float>(lr + k4, lv);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s4[k] += lv[k] * scr[(J << 8) + (k4 + k) * 16 + tx];
+        }
+        Li[(16 * I + ty) * kTileLd + 16 * J + tx] = -((s4[0] + s4[1]) + (s4[2] + s4[3]));
+      }
+      bar_sync(kBarB, 256);
+    }
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) A[ty * 4 + i][tx * 4 + j] = a[i][j];
-  // L^-1 and y_kb come from the diagonal factor launched just before this
-  // kernel (programmatic dependent launch): wait for its completion
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  load_tile_cg<T>(Li, Linv_all + (int64_t)kb * NB * NB, tid);
-  if (tid < NB) y[tid] = __ldcg(b + c0 + tid);
   __syncthreads();
-  T acc[4][4] = {};
-  tile_xyt<T>(A, Li, ty, tx, acc);
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    st4<T>(S + (r0 + ty * 4 + i) * ld + c0 + tx * 4, acc[i]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) A[ty * 4 + i][tx * 4 + j] = acc[i][j];
-  }
-  __syncthreads();
-  // b_ib -= L y: 4 threads per row, 16 columns each
-  {
+  // y = L^-1 b (4 threads per row); L^-1 and y out; L_ib,kb = S_ib,kb L^-T into T1
+  if (tid < 256) {
     const int r = tid >> 2, q = tid & 3;
-    T s4 = T(0);
+    float v = 0.f;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) s4 += A[r][16 * q + c] * y[16 * q + c];
+    for (int c = 0; c < 16; ++c) v += Li[r * kTileLd + 16 * q + c] * yb[16 * q + c];
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if (q == 0) {
+      yv[r] = v;
+      if (blockIdx.x == 0) y[off + r] = v;
+    }
+  }
+  if (blockIdx.x == 0) {
+    float* Lo = Linv_all + (int64_t)kb * NB * NB;
+    for (int idx = tid; idx < NB * NB / 4; idx += kPanel32Threads) {
+      float v[4];
+      ld4<float>(Li + (idx >> 4) * kTileLd + (idx & 15) * 4, v);
+      st4<float>(Lo + 4 * idx, v);
+    }
+  }
+  if (!has_tile) return;
+  {
+    const int ty = tid >> 4, tx = tid & 15;  // rows ty, ty + 32; columns tx + 16 j
+    float acc[2][4] = {};
+#pragma unroll 4
+    for (int k4 = 0; k4 < NB; k4 += 4) {
+      float x[2][4], z[4][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ld4<float>(T2 + (ty + 32 * i) * kTileLd + k4, x[i]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ld4<float>(Li + (tx + 16 * j) * kTileLd + k4, z[j]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[i][j] += x[i][k] * z[j][k];
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) T1[(ty + 32 * i) * kTileLd + tx + 16 * j] = acc[i][j];
+  }
+  __syncthreads();
+  for (int idx = tid; idx < NB * NB / 4; idx += kPanel32Threads) {
+    const int r = idx >> 4, c4 = idx & 15;
+    float v[4];
+    ld4<float>(T1 + r * kTileLd + 4 * c4, v);
+    st4<float>(S + (r0 + r) * ld + off + 4 * c4, v);
+    if (ops) {
+      float hi[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        hi[e] = umma::tf32_round(v[e]);
+        lo[e] = v[e] - hi[e];
+      }
+      float* d = ops + ib * kOpsTile + (c4 >> 3) * kOpsPiece + r * 32 + (((c4 & 7) ^ (r & 7)) << 2);
+      st4<float>(d, hi);
+      st4<float>(d + 2 * kOpsPiece, lo);
+    }
+  }
+  // b_ib -= L y: 4 threads per row, 16 columns each
+  if (tid < 256) {
+    const int r = tid >> 2, q = tid & 3;
+    float s4 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) s4 += T1[r * kTileLd + 16 * q + c] * yv[16 * q + c];
     s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
     s4 += __shfl_xor_sync(0xffffffffu, s4, 2);
-    if (q == 0) b[r0 + r] = __ldcg(b + r0 + r) - s4;
+    if (q == 0) b[r0 + r] -= s4;
   }
 }
 
@@ -557,55 +512,126 @@ __global__ void __launch_bounds__(256) k_syrk_wide(T* __restrict__ S, int64_t ld
     }
 }
 
-// The same trailing update on the tensor cores (FP32 path): one CTA per
-// 128 x 128 output tile of the same enumeration as k_syrk_wide, acc = X_i X_j^T
-// over the panel's 64 columns by tcgen05 kind::tf32 MMAs in 3xTF32 (FP32
-// accuracy), accumulated in tensor memory; the epilogue subtracts it from S.
-// Rows of a tile beyond the matrix edge are staged as zeros and not stored;
-// quarters above the diagonal are not stored.  A bounded wait that runs out
-// sets *flag = 6 (the step is then rejected) and the tile is left alone.
+// The same trailing update on the tensor cores (FP32 path): one CTA per 128 x
+// 64 output (two row tiles I >= J and the column tile J), acc = L_I L_J^T over
+// the panel's 64 columns by tcgen05 kind::tf32 MMAs in 3xTF32 (FP32 accuracy),
+// accumulated in tensor memory; the epilogue subtracts it from S.  The
+// operands' hi and lo parts were laid out by k_panel32 (once per tile instead
+// of once per output tile) and arrive by bulk copies; S's rows are loaded while
+// they do.  Two CTAs share an SM, so that one's copies and epilogue run beside
+// the other's.  Bound by S's traffic: the medium workload's first update moves
+// 144 MB of S and takes 40 us (91 us with 128 x 128 tiles that split their
+// own operands).
+// A bounded wait that runs out sets *flag = 6 (the step is then rejected) and
+// the tile is left alone.
+struct TcSmem {  // 1024-byte aligned (kTcSmem leaves room for it)
+  float a[4][2 * kOpsPiece];  // [hi, lo][32 columns], the two row tiles one after the other
+  float b[4][kOpsPiece];
+  uint64_t load_bar, mma_bar;
+  uint32_t tmem_base, fail;
+};
+constexpr size_t kTcSmem = sizeof(TcSmem) + 1024;
 constexpr int kSyrkTcThreads = 256;
-__global__ void __launch_bounds__(kSyrkTcThreads) k_syrk_tc(float* __restrict__ S, int64_t ld, int kb, int first,
-                                                            int nb, int* __restrict__ flag) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  umma::GemmSmem& g = *reinterpret_cast<umma::GemmSmem*>(smem_raw);
-  const int64_t t = blockIdx.x;
-  int64_t R = (int64_t)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-  while ((R + 1) * (R + 2) / 2 <= t) ++R;
-  while (R * (R + 1) / 2 > t) --R;
-  const int64_t C = t - R * (R + 1) / 2;
-  const int64_t ib0 = first + 2 * R, jb0 = first + 2 * C;
-  const int rows_i = ib0 + 1 < nb ? 2 * NB : NB, rows_j = jb0 + 1 < nb ? 2 * NB : NB;
-  const int64_t c0 = (int64_t)kb * NB;
-  umma::gemm_setup(g, 128);
-  const bool ok = umma::gemm_tile<kSyrkTcThreads>(g, 0, S + ib0 * NB * ld + c0, ld, S + jb0 * NB * ld + c0, ld, NB / umma::kChunk,
-                                  rows_i, rows_j);
-  if (ok) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = 32 * (w & 3) + lane;       // tile row = tensor-memory lane
-    const int qj = w >> 2;                   // column half: 64-tile jb0 + qj
-    const int64_t rb = ib0 + (r >> 6), cb = jb0 + qj;
-    if (rb < nb && cb < nb && rb >= cb) {
-      float* row = S + (rb * NB + (r & 63)) * ld + cb * NB;
+__global__ void __launch_bounds__(kSyrkTcThreads, 2) k_syrk_tc(float* __restrict__ S, int64_t ld, int j0, int nb,
+                                                               const float* __restrict__ ops, int* __restrict__ flag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TcSmem& g = *reinterpret_cast<TcSmem*>(smem_raw + ((1024 - (umma::smem_addr(smem_raw) & 1023)) & 1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // CTA t: column tile jb = j0, j0 + 1, ... with ceil((nb - jb) / 2) pairs of row tiles each
+  int jb = j0, t = blockIdx.x;
+  while (t >= (nb - jb + 1) / 2) {
+    t -= (nb - jb + 1) / 2;
+    ++jb;
+  }
+  const int ib = jb + 2 * t;
+  const bool two = ib + 1 < nb;
+  if (tid == 0) {
+    umma::mbar_init(&g.load_bar, 1);
+    umma::mbar_init(&g.mma_bar, 1);
+    g.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    constexpr uint32_t kBytes = kOpsPiece * 4;
+    const float* pa = ops + ib * (int64_t)kOpsTile;
+    const float* pb = ops + jb * (int64_t)kOpsTile;
+    umma::mbar_expect(&g.load_bar, (two ? 12 : 8) * kBytes);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float v[32];
-        umma::tmem_ld32(g.tmem_base + ((uint32_t)(32 * (w & 3)) << 16) + 64 * qj + 32 * h, v);
+    for (int p = 0; p < 4; ++p) {
+      umma::bulk_load(g.a[p], pa + p * kOpsPiece, kBytes, &g.load_bar);
+      if (two) umma::bulk_load(g.a[p] + kOpsPiece, pa + kOpsTile + p * kOpsPiece, kBytes, &g.load_bar);
+      umma::bulk_load(g.b[p], pb + p * kOpsPiece, kBytes, &g.load_bar);
+    }
+  }
+  if (warp == 0) {
+    __syncwarp();
+    umma::tmem_alloc(&g.tmem_base, 64);
+    umma::tmem_relinquish();
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tm = g.tmem_base;
+  // S: thread t takes 16-byte pieces t, t + 256, ... of the rows (16 a row)
+  float* out = S + (int64_t)ib * NB * ld + (int64_t)jb * NB + 4 * (tid & 15);
+  const int rows = two ? 2 * NB : NB;
+  float4 x[8];
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float4 c = *reinterpret_cast<float4*>(row + 32 * h + e);
-          c.x -= v[e];
-          c.y -= v[e + 1];
-          c.z -= v[e + 2];
-          c.w -= v[e + 3];
-          *reinterpret_cast<float4*>(row + 32 * h + e) = c;
-        }
+  for (int e = 0; e < 8; ++e) {
+    const int r = (tid >> 4) + 16 * e;
+    if (r < rows) x[e] = *reinterpret_cast<const float4*>(out + (int64_t)r * ld);
+  }
+  if (tid == 0) {
+    constexpr uint32_t idesc = umma::idesc_tf32(128, 64);
+    const uint64_t da = umma::smem_desc_sw128(umma::smem_addr(g.a[0]));
+    const uint64_t db = umma::smem_desc_sw128(umma::smem_addr(g.b[0]));
+    constexpr uint32_t kA = sizeof(g.a[0]) / 16, kB = sizeof(g.b[0]) / 16;
+    const bool ok = umma::mbar_wait(&g.load_bar, 0);
+    if (ok) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {  // 8 columns: piece k / 4, 32 bytes each
+        const uint32_t ca = (k >> 2) * kA + 2 * (k & 3), cb = (k >> 2) * kB + 2 * (k & 3);
+        umma::mma_tf32(tm, da + 2 * kA + ca, db + cb, idesc, k != 0);  // lo hi
+        umma::mma_tf32(tm, da + ca, db + 2 * kB + cb, idesc, 1);       // hi lo
+        umma::mma_tf32(tm, da + ca, db + cb, idesc, 1);                // hi hi
       }
-    }  // (the condition is uniform over a warp, as the warp-collective tcgen05.ld requires)
-  } else if (threadIdx.x == 0) {
+    }
+    umma::mma_commit(&g.mma_bar);
+    if (!umma::mbar_wait(&g.mma_bar, 0) || !ok) g.fail = 1;
+  }
+  __syncthreads();  // one thread polls, the others wait here
+  const bool ok = g.fail == 0;
+  umma::fence_after_sync();
+  if (ok) {
+    // accumulator rows (a tensor-memory lane each) through shared memory to
+    // the threads that hold S's pieces
+    constexpr int kLd = NB + 4;
+    float* acc = g.a[0];
+    {
+      float v[32];
+      const int r = 32 * (warp & 3) + lane, c0 = 32 * (warp >> 2);
+      umma::tmem_ld32(tm + ((uint32_t)(32 * (warp & 3)) << 16) + c0, v);
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) st4<float>(acc + r * kLd + c0 + e, v + e);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int r = (tid >> 4) + 16 * e;
+      if (r >= rows) continue;
+      float v[4];
+      ld4<float>(acc + r * kLd + 4 * (tid & 15), v);
+      x[e].x -= v[0];
+      x[e].y -= v[1];
+      x[e].z -= v[2];
+      x[e].w -= v[3];
+      *reinterpret_cast<float4*>(out + (int64_t)r * ld) = x[e];
+    }
+  } else if (tid == 0) {
     atomicExch(flag, 6);
   }
-  umma::gemm_teardown(g, 128);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  if (warp == 0) umma::tmem_dealloc(tm, 64);
 }
 
 template <typename T>
@@ -1178,9 +1204,11 @@ __global__ void __launch_bounds__(256) k_tile_inverse(double* __restrict__ Linv_
 }
 constexpr size_t kTileInverseSmem = sizeof(double) * (2 * 64 * kPanelLd + 3 * 256);
 
-// Bytes of the FP64 factorisation's workspace: the digits of two panels (the
-// trailing update of a panel runs beside the next) with their rows' exponents, and y.
-size_t dense_cholesky_work_bytes(int64_t n_pad) {
+// Bytes of the factorisation's workspace: the operands of two panels (the
+// trailing update of a panel runs beside the next; FP64: digits and their
+// rows' exponents), and y.
+size_t dense_cholesky_work_bytes(int64_t n_pad, bool fp64) {
+  if (!fp64) return 2 * (size_t)(n_pad / NB) * kOpsTile * sizeof(float) + (size_t)n_pad * sizeof(float);
   return 2 * (size_t)(n_pad / NB) * kTileDigitBytes + (size_t)n_pad * (sizeof(double) + 2 * sizeof(int32_t));
 }
 
@@ -1193,13 +1221,10 @@ void dense_cholesky_prepare() {
     const int sm = (int)dense_smem_bytes<T>();
     GBBA_CUDA(cudaFuncSetAttribute(k_trsv_bwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     if constexpr (std::is_same<T, float>::value) {
-      GBBA_CUDA(cudaFuncSetAttribute(k_potrf_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)potrf_smem_bytes<T>()));
-      GBBA_CUDA(cudaFuncSetAttribute(k_trsm_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+      GBBA_CUDA(cudaFuncSetAttribute(k_panel32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanel32Smem));
       GBBA_CUDA(cudaFuncSetAttribute(k_syrk_wide<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)wide_smem_bytes<T>()));
-      GBBA_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(umma::GemmSmem)));
+      GBBA_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     } else {
       GBBA_CUDA(cudaFuncSetAttribute(k_panel64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)panel64_smem(kPanelMaxRows)));
@@ -1239,62 +1264,57 @@ void launch_hi(gbba_handle* h, bool pdl, void (*k)(Exp...), unsigned grid, unsig
   count_launch(h);
 }
 
-// Solve S x = b in place of (S -> L, b -> y); x receives the solution.
+// Solve S x = b (S -> L below the diagonal tiles, b is used up); x receives
+// the solution.
 //
 // Right-looking, 64-wide panels, look-ahead by one panel.  Per step k the
-// call's stream runs two kernels:
-//   potrf(k+1): applies panel k's update to diagonal tile k+1, factors it
-//               (L, L^-1, y_{k+1});
-//   trsm(k+1):  applies panel k's update to the tiles below it in block
-//               column k+1, then solves them (and updates b);
-// while the side stream applies panel k's update to block columns k+2..
-// (128-wide tiles).  The two streams touch disjoint tiles; the call's stream
-// waits for the side stream's step k-1 before step k (that step wrote block
-// column k+1), and the side stream starts step k once panel k is solved.
-// The side stream is joined back before the backward substitution, so the
-// sequence can be captured.
-// kTensor: the trailing update on the tensor cores (k_syrk_tc, FP32 only) or
-// on the FP32 pipes (k_syrk_wide).
-template <typename T, bool kTensor>
-void dense_cholesky_solve_impl(gbba_handle* h, T* S, int64_t n_pad, T* b, T* x, T* Linv_all, int* flag,
-                               cudaStream_t st) {
+// call's stream runs panel(k+1), which applies panel k's update to block
+// column k+1 itself and factors it, while the side stream applies panel k's
+// update to block columns k+2...  The two touch disjoint tiles; the call's
+// stream waits for the side stream's step k-1 before step k (that step wrote
+// block column k+1 and read the operands that panel k+1 replaces), and the
+// side stream starts step k once panel k is solved.  The side stream is joined
+// back before the backward substitution, so the sequence can be captured.
+// tensor: the trailing update on the tensor cores (k_syrk_tc) or on the FP32
+// pipes (k_syrk_wide).
+static void dense_cholesky_solve_fp32(gbba_handle* h, float* S, int64_t n_pad, float* b, float* x, float* Linv_all,
+                                      void* work, int* flag, cudaStream_t st, bool tensor) {
   const int nb = (int)(n_pad / NB);
-  const size_t sm = dense_smem_bytes<T>(), psm = potrf_smem_bytes<T>();
-  dense_cholesky_prepare<T>();
-  launch_hi(h, false, k_potrf_diag<T>, 1, kPotrfThreads, psm, st, S, n_pad, 0, Linv_all, b, flag, 0);
-  if (nb > 1)
-    launch_hi(h, true, k_trsm_panel<T>, (unsigned)(nb - 1), 256, sm, st, S, n_pad, 0, (const T*)Linv_all, b, 0);
+  dense_cholesky_prepare<float>();
+  float* const ops[2] = {static_cast<float*>(work), static_cast<float*>(work) + (int64_t)nb * kOpsTile};
+  float* y = ops[1] + (int64_t)nb * kOpsTile;
   bool side_pending = false;
-  for (int k = 0; k + 1 < nb; ++k) {
+  for (int k = -1; k + 1 < nb; ++k) {
     const int rem = nb - k - 1;  // tiles in block column k+1, diagonal included
     if (side_pending) {
       GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
       side_pending = false;
     }
-    if (rem > 1) {
+    if (k >= 0 && rem > 1) {
       GBBA_CUDA(cudaEventRecord(h->ev_main, st));
       GBBA_CUDA(cudaStreamWaitEvent(h->side, h->ev_main, 0));
-      const int64_t tw = rem / 2;  // 128-tiles per side over the 64-tiles k+2..nb-1
-      if constexpr (kTensor)
-        k_syrk_tc<<<(unsigned)(tw * (tw + 1) / 2), kSyrkTcThreads, sizeof(umma::GemmSmem), h->side>>>(
-            S, n_pad, k, k + 2, nb, flag);
-      else
-        k_syrk_wide<T><<<(unsigned)(tw * (tw + 1) / 2), 256, wide_smem_bytes<T>(), h->side>>>(S, n_pad, k, k + 2, nb);
+      if (tensor) {
+        int64_t ctas = 0;
+        for (int j = k + 2; j < nb; ++j) ctas += (nb - j + 1) / 2;
+        k_syrk_tc<<<(unsigned)ctas, kSyrkTcThreads, kTcSmem, h->side>>>(S, n_pad, k + 2, nb, ops[k & 1], flag);
+      } else {
+        const int64_t tw = rem / 2;  // 128-tiles per side over the 64-tiles k+2..nb-1
+        k_syrk_wide<float><<<(unsigned)(tw * (tw + 1) / 2), 256, wide_smem_bytes<float>(), h->side>>>(S, n_pad, k,
+                                                                                                      k + 2, nb);
+      }
       check_launch(h);
       GBBA_CUDA(cudaEventRecord(h->ev_side, h->side));
       side_pending = true;
     }
-    launch_hi(h, false, k_potrf_diag<T>, 1, kPotrfThreads, psm, st, S, n_pad, k + 1, Linv_all, b, flag, 1);
-    if (rem > 1)
-      launch_hi(h, true, k_trsm_panel<T>, (unsigned)(rem - 1), 256, sm, st, S, n_pad, k + 1, (const T*)Linv_all,
-                b, 1);
+    launch_hi(h, false, k_panel32, (unsigned)std::max(1, rem - 1), kPanel32Threads, kPanel32Smem, st, S, n_pad, k + 1,
+              nb, Linv_all, b, y, tensor ? ops[(k + 1) & 1] : nullptr, flag);
   }
   if (side_pending) GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
   // backward substitution: each block row's kernel starts while the previous
   // one finishes (programmatic dependent launch; the first one waits fully)
   for (int kb = nb - 1; kb >= 0; --kb)
-    launch_hi(h, kb != nb - 1, k_trsv_bwd<T>, (unsigned)(kb + 1), 256, sm, st, S, n_pad, kb,
-              (const T*)Linv_all, b, x);
+    launch_hi(h, kb != nb - 1, k_trsv_bwd<float>, (unsigned)(kb + 1), 256, dense_smem_bytes<float>(), st,
+              (const float*)S, n_pad, kb, (const float*)Linv_all, y, x);
 }
 
 // FP64: the same look-ahead with the kernels above.  Per step k the call's
@@ -1346,23 +1366,16 @@ static void dense_cholesky_solve_fp64(gbba_handle* h, double* S, int64_t n, int6
               (const double*)S, n_pad, kb, (const double*)Linv_all, y, x);
 }
 
-// n: unknowns of S (n_pad with the padding); work: dense_cholesky_work_bytes
-// (FP64 only).
+// n: unknowns of S (n_pad with the padding); work: dense_cholesky_work_bytes.
 template <typename T>
 void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n, int64_t n_pad, T* b, T* x, T* Linv_all, void* work,
                           int* flag, cudaStream_t st) {
   if constexpr (std::is_same<T, double>::value)
     dense_cholesky_solve_fp64(h, S, n, n_pad, b, x, Linv_all, work, flag, st);
-  else if (h->factor_tensor)
-    dense_cholesky_solve_impl<T, true>(h, S, n_pad, b, x, Linv_all, flag, st);
   else
-    dense_cholesky_solve_impl<T, false>(h, S, n_pad, b, x, Linv_all, flag, st);
+    dense_cholesky_solve_fp32(h, S, n_pad, b, x, Linv_all, work, flag, st, h->factor_tensor);
 }
 
-template void dense_cholesky_solve_impl<float, false>(gbba_handle*, float*, int64_t, float*, float*, float*, int*,
-                                                      cudaStream_t);
-template void dense_cholesky_solve_impl<float, true>(gbba_handle*, float*, int64_t, float*, float*, float*, int*,
-                                                     cudaStream_t);
 template void dense_cholesky_prepare<double>();
 template void dense_cholesky_prepare<float>();
 template void dense_cholesky_solve<double>(gbba_handle*, double*, int64_t, int64_t, double*, double*, double*, void*,

@@ -44,7 +44,7 @@ namespace gbba {
 template <typename T>
 void dense_cholesky_solve(gbba_handle* h, T* S, int64_t n, int64_t n_pad, T* b, T* x, T* Linv_all, void* work,
                           int* flag, cudaStream_t st);
-size_t dense_cholesky_work_bytes(int64_t n_pad);
+size_t dense_cholesky_work_bytes(int64_t n_pad, bool fp64);
 template <typename T>
 void dense_cholesky_prepare();
 
@@ -2778,7 +2778,7 @@ static void carve(A& a, Solve& s, size_t tsize) {
   s.rhs = a.template take<char>((size_t)s.n_pad * tsize);
   s.zsol = a.template take<char>((size_t)s.n_pad * tsize);
   s.Linv = a.template take<char>((size_t)n_s * kDenseTile * tsize);
-  s.cwork = a.template take<char>(tsize == 8 ? dense_cholesky_work_bytes(n_s) : 0);
+  s.cwork = a.template take<char>(dense_cholesky_work_bytes(n_s, tsize == 8));
   s.Vinv = a.template take<char>((size_t)s.np * 6 * tsize);
   s.gpv = a.template take<char>((size_t)s.np * 3 * tsize);
   s.part_mcc = a.template take<double>(s.nb_pt);

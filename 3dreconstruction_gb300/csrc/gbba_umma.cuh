@@ -3,13 +3,10 @@
 // accumulation in tensor memory, completion through an mbarrier, and the
 // tensor-memory loads of the epilogue.  Written as inline PTX.
 //
-// Operand layout (both operands K-major, no swizzle): a 128 x KC tile is a
-// grid of "core matrices" of 8 rows x 16 bytes (4 FP32 values per row, rows
-// 16 bytes apart, 128 bytes per core matrix).  Core matrix (r8, k4) sits at
-// byte ((r8 * KC / 4) + k4) * 128 from the tile base, so core matrices that
-// are neighbours along K are 128 bytes apart (the descriptor's leading
-// dimension byte offset) and neighbours along M/N are KC * 32 bytes apart
-// (its stride dimension byte offset).
+// Operand layout (both operands K-major, 128-byte swizzle): rows of 128 bytes
+// (32 FP32 or 64 FP16 values), eight rows a swizzle atom of 1024 bytes (1024-
+// byte aligned), the 16-byte chunk c of row r stored at chunk c ^ (r % 8),
+// atoms 1024 bytes apart along M/N.
 //
 // FP32 accuracy from TF32 inputs (3xTF32): every operand value x is split as
 // x = hi + lo with hi = x rounded to TF32 and lo = x - hi (exact in FP32),
@@ -39,10 +36,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Generic-proxy shared-memory stores become visible to the tensor core's
-// (async-proxy) operand reads.
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
@@ -64,18 +57,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
-// Shared-memory matrix descriptor: start address, leading (K) and stride
-// (M/N) byte offsets between core matrices, descriptor version 1, no swizzle.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
-// The same for K-major operands in 128-byte swizzle: rows of 128 bytes, eight
-// rows (1024 bytes, aligned) a swizzle atom, the 16-byte chunk c of row r at
-// chunk c ^ (r % 8), atoms 1024 bytes apart along M/N.  32 bytes of K on is
-// the start address + 32.  (Without the swizzle an MMA reads a 128-row operand
-// at 30 bytes a clock: 138 clocks for M = 128, K = 32 bytes, whatever N.)
+// Shared-memory matrix descriptor: start address, stride byte offset between
+// atoms along M/N (1024), descriptor version 1, 128-byte swizzle.  32 bytes of
+// K on is the start address + 32.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
@@ -165,134 +149,6 @@ __device__ __forceinline__ float tf32_round(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return __uint_as_float(r);
-}
-
-// ------------------------------------------------------------------ 128 x 128 tile GEMM, K in chunks of 32
-constexpr int kTile = 128;
-constexpr int kChunk = 32;
-constexpr int kOperandFloats = kTile * kChunk;  // one 128 x 32 operand tile (16 KB)
-
-// Shared memory of one tile GEMM: hi and lo parts of the A and B chunks, the
-// completion barrier and the tensor-memory base address.
-struct GemmSmem {
-  float a_hi[kOperandFloats], a_lo[kOperandFloats], b_hi[kOperandFloats], b_lo[kOperandFloats];
-  uint64_t bar;
-  uint32_t tmem_base;
-  uint32_t phase;
-};
-
-// Core-layout offset (in floats) of row r, columns 4q..4q+3 of a 128 x 32 chunk.
-__device__ __forceinline__ int core_offset(int r, int q) { return ((r >> 3) * (kChunk / 4) + q) * 32 + (r & 7) * 4; }
-
-// One thread's share of a 128 x 32 chunk of a row-major FP32 block: with T
-// threads, thread t loads float4 number t, t + T, ... (row idx / 8, columns
-// 4 (idx % 8)..), kPer of them.  The loads are issued together (prefetch) and
-// stored as hi / lo parts in core layout later (commit), so that a chunk's
-// global-memory latency overlaps the previous chunk's MMAs.
-template <int kThreads>
-struct ChunkRegs {
-  static constexpr int kPer = kTile * kChunk / 4 / kThreads;
-  float4 v[kPer];
-  __device__ __forceinline__ void prefetch(const float* __restrict__ src, int64_t ld, int k0, int valid_rows, int tid) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int idx = tid + u * kThreads, r = idx >> 3, q = idx & 7;
-      v[u] = r < valid_rows ? __ldcg(reinterpret_cast<const float4*>(src + (int64_t)r * ld + k0 + 4 * q))
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  __device__ __forceinline__ void commit(float* hi, float* lo, int tid) const {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int idx = tid + u * kThreads, r = idx >> 3, q = idx & 7;
-      float4 h, l;
-      h.x = tf32_round(v[u].x); l.x = v[u].x - h.x;
-      h.y = tf32_round(v[u].y); l.y = v[u].y - h.y;
-      h.z = tf32_round(v[u].z); l.z = v[u].z - h.z;
-      h.w = tf32_round(v[u].w); l.w = v[u].w - h.w;
-      const int o = core_offset(r, q);
-      *reinterpret_cast<float4*>(hi + o) = h;
-      *reinterpret_cast<float4*>(lo + o) = l;
-    }
-  }
-};
-
-// Set-up by the whole CTA (warp 0 allocates `ncols` tensor-memory columns).
-__device__ __forceinline__ void gemm_setup(GemmSmem& g, uint32_t ncols) {
-  if (threadIdx.x == 0) {
-    mbar_init(&g.bar, 1);
-    g.phase = 0;
-  }
-  if (threadIdx.x < 32) {
-    tmem_alloc(&g.tmem_base, ncols);
-    tmem_relinquish();
-  }
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-}
-__device__ __forceinline__ void gemm_teardown(GemmSmem& g, uint32_t ncols) {
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  if (threadIdx.x < 32) tmem_dealloc(g.tmem_base, ncols);
-}
-
-// acc (tensor memory, columns col0..col0+127) = A B^T over K = 32 * nchunks,
-// A and B 128-row row-major FP32 blocks (row strides lda, ldb), 3xTF32; rows
-// at or beyond a_rows / b_rows are taken as zero (and not read).  All
-// kThreads threads of the CTA call it.  The next chunk's loads are in flight
-// while the tensor core works on the current one.  Returns false when a
-// bounded wait for the tensor core ran out (the caller records the error).
-template <int kThreads>
-__device__ __forceinline__ bool gemm_tile(GemmSmem& g, uint32_t col0, const float* __restrict__ A, int64_t lda,
-                                          const float* __restrict__ B, int64_t ldb, int nchunks, int a_rows = kTile,
-                                          int b_rows = kTile) {
-  const int tid = threadIdx.x;
-  constexpr uint32_t idesc = idesc_tf32(kTile, kTile);
-  constexpr uint32_t LBO = 128, SBO = kChunk * 32;
-  ChunkRegs<kThreads> ra, rb;
-  ra.prefetch(A, lda, 0, a_rows, tid);
-  rb.prefetch(B, ldb, 0, b_rows, tid);
-  bool ok = true;
-  for (int c = 0; c < nchunks; ++c) {
-    if (c > 0) {
-      // the MMAs of chunk c-1 read the staging buffers asynchronously: wait
-      // for them before the buffers are overwritten
-      ok = __syncthreads_and(mbar_wait(&g.bar, g.phase) && ok) != 0;
-      if (tid == 0) g.phase ^= 1u;
-      fence_after_sync();
-      if (!ok) break;
-    }
-    ra.commit(g.a_hi, g.a_lo, tid);
-    rb.commit(g.b_hi, g.b_lo, tid);
-    if (c + 1 < nchunks) {
-      ra.prefetch(A, lda, (c + 1) * kChunk, a_rows, tid);
-      rb.prefetch(B, ldb, (c + 1) * kChunk, b_rows, tid);
-    }
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      fence_after_sync();
-      const uint32_t ah = smem_addr(g.a_hi), al = smem_addr(g.a_lo), bh = smem_addr(g.b_hi), bl = smem_addr(g.b_lo);
-#pragma unroll
-      for (int kk = 0; kk < kChunk / 8; ++kk) {
-        const uint32_t o = kk * 2 * 128;  // two core matrices (8 TF32 values) along K per MMA
-        mma_tf32(g.tmem_base + col0, smem_desc(al + o, LBO, SBO), smem_desc(bh + o, LBO, SBO), idesc,
-                 (c | kk) != 0);
-        mma_tf32(g.tmem_base + col0, smem_desc(ah + o, LBO, SBO), smem_desc(bl + o, LBO, SBO), idesc, 1);
-        mma_tf32(g.tmem_base + col0, smem_desc(ah + o, LBO, SBO), smem_desc(bh + o, LBO, SBO), idesc, 1);
-      }
-      mma_commit(&g.bar);
-    }
-  }
-  if (ok) {
-    ok = __syncthreads_and(mbar_wait(&g.bar, g.phase)) != 0;
-    if (tid == 0) g.phase ^= 1u;
-    fence_after_sync();
-    __syncthreads();
-  }
-  return ok;
 }
 
 }  // namespace umma

@@ -1,10 +1,11 @@
-"""FP64 dense factorisation (panels on the FP64 pipe, trailing update by exact
+"""Dense factorisation, FP64 (panels on the FP64 pipe, trailing update by exact
 FP16 digit products on the tensor cores): reduced systems on both sides of its
 16-column blocks, 64-column panels and 128-row tile pairs, and one with
 several panels of look-ahead, against the CPU oracle.  The step solves a
 system of condition up to about 1e6 in FP64 arithmetic, so the parameters
 after a few iterations agree to 1e-8 and the costs to 1e-9 relative, the
-tolerances of the other FP64 comparisons with the oracle."""
+tolerances of the other FP64 comparisons with the oracle.  The FP32
+factorisation of the mixed path is checked on the same sizes."""
 import numpy as np
 import pytest
 
@@ -23,6 +24,21 @@ def test_panel_edges_match_oracle(model, cameras, handle, abi, scenes, oracle_mo
     assert s.usable and s.num_iterations == so["num_iterations"]
     assert abs(s.final_cost - so["final_cost"]) <= 1e-9 * so["final_cost"]
     np.testing.assert_allclose(hp.points.reshape(-1, 3), np.asarray(po["points"]).reshape(-1, 3), rtol=0, atol=1e-8)
+
+
+@pytest.mark.parametrize("cameras", [3, 6, 11, 12, 17, 22, 45])
+def test_mixed_panel_edges_reach_fp64_cost(cameras, handle, abi, scenes):
+    """The FP32 panel and TF32 trailing update on the same sizes: the mixed
+    solve ends at the FP64 solve's cost (1e-6 relative, the mixed path's bar)."""
+    sc = scenes.medium_scene(num_cameras=cameras, num_points=40 * cameras, mean_views=min(5, cameras - 2),
+                             seed=330 + cameras, hold=(0, 1))
+    cost = {}
+    for p in (abi.PRECISION_FP64, abi.PRECISION_MIXED):
+        hp = abi.HostProblem(sc)
+        s = handle.solve(hp, scenes.ba_options_for(sc, max_num_iterations=100, precision=p))
+        assert s.usable
+        cost[p] = s.final_cost
+    assert cost[abi.PRECISION_MIXED] <= cost[abi.PRECISION_FP64] * (1 + 1e-6)
 
 
 def test_indefinite_system_is_rejected(handle, abi, scenes):
