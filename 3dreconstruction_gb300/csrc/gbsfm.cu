@@ -345,92 +345,127 @@ enum : unsigned long long {
   kBadCameraImage = 32 // a write-back ordinal names an image outside the state
 };
 
-// Exclusive block-wide count of `flag` over blockDim.x <= 1024 threads;
-// returns the thread's offset and leaves the block total in *total.
-__device__ __forceinline__ uint32_t block_exclusive_count(bool flag, uint32_t* sh_warp, uint32_t* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  const unsigned mask = __ballot_sync(0xffffffffu, flag);
-  if (lane == 0) sh_warp[warp] = __popc(mask);
+// Reconstructed images in chunks of kImageChunk (the camera ordinals' bases).
+constexpr int kImageChunk = 8192;
+constexpr int kImageThreads = 128;
+__device__ __forceinline__ uint32_t block_total(uint32_t v, uint32_t* sh) {  // kImageThreads threads
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();  // sh is reused
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  uint32_t before = 0, all = 0;
-  for (int w = 0; w < nw; ++w) {
-    const uint32_t c = sh_warp[w];
-    before += w < warp ? c : 0u;
-    all += c;
-  }
-  __syncthreads();  // sh_warp is reused by the next call
-  *total = all;
-  return before + __popc(mask & ((1u << lane) - 1u));
+  uint32_t t = 0;
+#pragma unroll
+  for (int w = 0; w < kImageThreads / 32; ++w) t += sh[w];
+  return t;
+}
+__global__ void __launch_bounds__(kImageThreads) k_image_counts(int64_t ni, const uint8_t* __restrict__ rec,
+                                                                uint32_t* __restrict__ chunk_count) {
+  __shared__ uint32_t sh[kImageThreads / 32];
+  const int64_t i0 = (int64_t)blockIdx.x * kImageChunk, i1 = min(ni, i0 + kImageChunk);
+  uint32_t n = 0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += kImageThreads) n += rec[i] != 0;
+  n = block_total(n, sh);
+  if (threadIdx.x == 0) chunk_count[blockIdx.x] = n;
 }
 
-// One block over the images: camera ordinals (ascending image id among the
+// What an entry of the pack needs of its image, in one 16-byte load: the place
+// of its first feature, their count (0 when the offsets are not a run inside
+// the features) and its intrinsic group.
+struct __align__(16) ImageRow {
+  int64_t first;
+  uint32_t count, group;
+};
+
+// One image per thread: camera ordinals (ascending image id among the
 // reconstructed, the key order of map_Camera), the extrinsic blocks
-// [angle-axis, t] and the ordinal -> image table.
-__global__ void __launch_bounds__(1024) k_pack_images(int64_t ni, const uint8_t* __restrict__ rec,
-                                                      const gbsfm_camera* __restrict__ cams,
-                                                      const uint32_t* __restrict__ group, int64_t num_groups,
-                                                      uint32_t* __restrict__ ordinal, double* __restrict__ ext,
-                                                      uint32_t* __restrict__ camera_image,
-                                                      unsigned long long* __restrict__ counters) {
-  __shared__ uint32_t sh_warp[32];
-  uint32_t base = 0;
-  unsigned long long err = 0;
-  for (int64_t c0 = 0; c0 < ni; c0 += blockDim.x) {
-    const int64_t i = c0 + threadIdx.x;
-    const bool flag = i < ni && rec[i] != 0;
-    uint32_t total;
-    const uint32_t pos = base + block_exclusive_count(flag, sh_warp, &total);
-    if (i < ni) ordinal[i] = flag ? pos : kNoCamera;
-    if (flag) {
-      const gbsfm_camera& c = cams[i];
-      double aa[3];
-      rotation_to_angle_axis(c.R, aa);
-      double* e = ext + 6 * (int64_t)pos;
-      e[0] = aa[0];
-      e[1] = aa[1];
-      e[2] = aa[2];
-      e[3] = c.t[0];
-      e[4] = c.t[1];
-      e[5] = c.t[2];
-      if (camera_image) camera_image[pos] = (uint32_t)i;
-      if (group[i] >= (uint64_t)num_groups) err |= kBadGroup;
-    }
-    base += total;
+// [angle-axis, t] and the ordinal -> image table.  A block's base is the count
+// of the chunks before its own (chunk_count; the first chunk needs none) and
+// of the flags before it in the chunk.  The conversions are FP64 (~200
+// operations an image at two a clock per SM), so they are spread over the SMs
+// by small blocks: 5,000 images 236 us in one block, 12 us in 40.
+__global__ void __launch_bounds__(kImageThreads) k_pack_images(int64_t ni, const uint8_t* __restrict__ rec,
+                                                               const gbsfm_camera* __restrict__ cams,
+                                                               const uint32_t* __restrict__ group, int64_t num_groups,
+                                                               const uint32_t* __restrict__ chunk_count,
+                                                               const int64_t* __restrict__ feature_offsets, int64_t nf,
+                                                               ImageRow* __restrict__ rows,
+                                                               uint32_t* __restrict__ ordinal, double* __restrict__ ext,
+                                                               uint32_t* __restrict__ camera_image,
+                                                               unsigned long long* __restrict__ counters) {
+  __shared__ uint32_t sh[kImageThreads / 32];
+  const int64_t i0 = (int64_t)blockIdx.x * kImageThreads, i = i0 + threadIdx.x;
+  const int64_t chunk = i0 / kImageChunk;
+  uint32_t before = 0;
+  for (int64_t c = threadIdx.x; c < chunk; c += kImageThreads) before += chunk_count[c];
+  for (int64_t k = chunk * kImageChunk + threadIdx.x; k < i0; k += kImageThreads) before += rec[k] != 0;
+  const uint32_t base = block_total(before, sh);
+  const bool flag = i < ni && rec[i] != 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, flag);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();
+  if (lane == 0) sh[warp] = __popc(mask);
+  __syncthreads();
+  uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) pos += sh[w];
+  if (i < ni) {
+    ordinal[i] = flag ? pos : kNoCamera;
+    const int64_t a = feature_offsets[i], b = feature_offsets[i + 1];
+    const bool ok = a >= 0 && b <= nf && b > a;
+    rows[i] = ImageRow{a, ok ? (uint32_t)min(b - a, (int64_t)0xffffffff) : 0u, group[i]};
   }
-  if (err) atomicOr(&counters[2], err);
-  if (threadIdx.x == 0) counters[0] = base;
+  if (flag) {
+    const gbsfm_camera& c = cams[i];
+    double aa[3];
+    rotation_to_angle_axis(c.R, aa);
+    double* e = ext + 6 * (int64_t)pos;
+    e[0] = aa[0];
+    e[1] = aa[1];
+    e[2] = aa[2];
+    e[3] = c.t[0];
+    e[4] = c.t[1];
+    e[5] = c.t[2];
+    if (camera_image) camera_image[pos] = (uint32_t)i;
+    if (group[i] >= (uint64_t)num_groups) atomicOr(&counters[2], (unsigned long long)kBadGroup);
+  }
+  if (i == ni - 1) counters[0] = pos + (flag ? 1 : 0);
 }
 
-__device__ __forceinline__ bool entry_kept(int64_t e, int64_t ne, int64_t ni, const uint32_t* __restrict__ img,
-                                           const uint32_t* __restrict__ ordinal, uint32_t* im) {
-  if (e >= ne) return false;
-  *im = img[e];
-  return *im < (uint64_t)ni && ordinal[*im] != kNoCamera;
-}
-
-// Pass 1 over the entries: kept entries per tile of 2048, and the checks of
-// the image ids and of the track offsets.
+// Pass 1 over the entries: kept entries per tile of 2048, the track of each
+// tile's first entry, and the checks of the image ids and of the track offsets.  Thread t takes entries 8t .. 8t+7
+// of the tile, in two 16-byte loads where the array is aligned for them.
 __global__ void __launch_bounds__(kPackThreads) k_pack_count(int64_t ne, int64_t ni, int64_t nt,
                                                              const int64_t* __restrict__ offs,
                                                              const uint32_t* __restrict__ img,
                                                              const uint32_t* __restrict__ ordinal,
                                                              uint32_t* __restrict__ tile_count,
+                                                             uint32_t* __restrict__ tile_track,
                                                              unsigned long long* __restrict__ counters) {
-  __shared__ uint32_t sh_warp[32];
+  __shared__ uint32_t sh_warp[kPackThreads / 32];
   unsigned long long err = 0;
   uint32_t kept = 0;
-  const int64_t tile = blockIdx.x * kPackTile;
+  const int64_t e0 = blockIdx.x * kPackTile + (int64_t)threadIdx.x * kPackPer;
+  uint32_t im[kPackPer];
+  static_assert(kPackPer == 8, "two 16-byte loads");
+  if (e0 + kPackPer <= ne && (reinterpret_cast<uintptr_t>(img) & 15) == 0) {
+    const uint4 a = *reinterpret_cast<const uint4*>(img + e0), b = *reinterpret_cast<const uint4*>(img + e0 + 4);
+    im[0] = a.x, im[1] = a.y, im[2] = a.z, im[3] = a.w, im[4] = b.x, im[5] = b.y, im[6] = b.z, im[7] = b.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPackPer; ++j) im[j] = e0 + j < ne ? img[e0 + j] : 0u;
+  }
 #pragma unroll
   for (int j = 0; j < kPackPer; ++j) {
-    const int64_t e = tile + j * kPackThreads + threadIdx.x;
-    uint32_t im = 0;
-    kept += entry_kept(e, ne, ni, img, ordinal, &im) ? 1u : 0u;
-    if (e < ne && im >= (uint64_t)ni) err |= kBadImage;
+    if (e0 + j >= ne) continue;
+    if (im[j] >= (uint64_t)ni) err |= kBadImage;
+    else kept += ordinal[im[j]] != kNoCamera ? 1u : 0u;
   }
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t <= nt; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t o = offs[t];
-    const bool bad = (t == 0 && o != 0) || (t == nt && o != ne) || (t < nt && offs[t + 1] < o);
+    const int64_t o = offs[t], next = t < nt ? offs[t + 1] : o;
+    const bool bad = (t == 0 && o != 0) || (t == nt && o != ne) || next < o || o < 0 || next > ne;
     if (bad) err |= kBadOffsets;
+    else
+      for (int64_t k = (o + kPackTile - 1) / kPackTile; k * kPackTile < next; ++k) tile_track[k] = (uint32_t)t;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
@@ -444,77 +479,157 @@ __global__ void __launch_bounds__(kPackThreads) k_pack_count(int64_t ne, int64_t
   if (err) atomicOr(&counters[2], err);
 }
 
-// Exclusive scan of the tile counts in place (one block); the total is the
-// observation count.
-__global__ void __launch_bounds__(1024) k_pack_scan(uint32_t* __restrict__ tile_count, int64_t nb,
-                                                    unsigned long long* __restrict__ counters) {
-  __shared__ uint32_t sh[1024];
-  __shared__ unsigned long long sh_base;
-  if (threadIdx.x == 0) sh_base = 0;
-  __syncthreads();
-  for (int64_t c0 = 0; c0 < nb; c0 += 1024) {
-    const int64_t i = c0 + threadIdx.x;
-    const uint32_t v = i < nb ? tile_count[i] : 0u;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int d = 1; d < 1024; d <<= 1) {  // Hillis-Steele inclusive scan
-      const uint32_t add = threadIdx.x >= d ? sh[threadIdx.x - d] : 0u;
-      __syncthreads();
-      sh[threadIdx.x] += add;
-      __syncthreads();
-    }
-    const unsigned long long base = sh_base;
-    if (i < nb) tile_count[i] = (uint32_t)(base + sh[threadIdx.x] - v);
-    __syncthreads();
-    if (threadIdx.x == 1023) sh_base = base + sh[1023];
-    __syncthreads();
+// Inclusive sum over a block of up to 1024 threads; *total: the block's.
+__device__ __forceinline__ uint32_t block_inclusive_sum(uint32_t v, uint32_t* sh_warp, uint32_t* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += u;
   }
-  if (threadIdx.x == 0) counters[1] = sh_base;
+  if (lane == 31) sh_warp[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t w = lane < nw ? sh_warp[lane] : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, w, d);
+      if (lane >= d) w += u;
+    }
+    sh_warp[lane] = w;
+  }
+  __syncthreads();
+  *total = sh_warp[nw - 1];
+  if (warp > 0) v += sh_warp[warp - 1];
+  __syncthreads();  // sh_warp is reused by the next call
+  return v;
 }
 
-// Pass 2: the same tiles in entry order; each kept entry gets its place from
-// the tile base and the block-wide count, and gathers its feature (float ->
-// double), camera ordinal, intrinsic group and track (binary search of the
-// offsets: the last track that starts at or before the entry).
-__global__ void __launch_bounds__(kPackThreads) k_pack_gather(
-    int64_t ne, int64_t ni, int64_t nt, int64_t nf, const int64_t* __restrict__ offs,
-    const uint32_t* __restrict__ img, const uint32_t* __restrict__ feat, const uint32_t* __restrict__ ordinal,
-    const uint32_t* __restrict__ group, const int64_t* __restrict__ feature_offsets,
-    const float* __restrict__ features, const uint32_t* __restrict__ tile_base, double* __restrict__ obs,
+// Exclusive scan of the tile counts in place (one block, a run of consecutive
+// counts per thread); the total is the observation count.
+__global__ void __launch_bounds__(1024) k_pack_scan(uint32_t* __restrict__ tile_count, int64_t nb,
+                                                    unsigned long long* __restrict__ counters) {
+  __shared__ uint32_t sh_warp[32];
+  const int64_t per = (nb + 1023) / 1024, i0 = min(nb, threadIdx.x * per), i1 = min(nb, i0 + per);
+  uint32_t sum = 0, total;
+  for (int64_t i = i0; i < i1; ++i) sum += tile_count[i];
+  uint32_t run = block_inclusive_sum(sum, sh_warp, &total) - sum;
+  for (int64_t i = i0; i < i1; ++i) {
+    const uint32_t v = tile_count[i];
+    tile_count[i] = run;
+    run += v;
+  }
+  if (threadIdx.x == 0) counters[1] = total;
+}
+
+// Pass 2: the same tiles; each kept entry gets its place from the tile base and
+// the block-wide count, and gathers its feature (float -> double), camera
+// ordinal, intrinsic group and track.  The track (the last one that starts at
+// or before the entry) comes from a running maximum over the tile: the tracks
+// that start inside it mark their first entry.  Bound by the gathers (an entry's image row and feature
+// are on lines of their own), so they are few and wide, and a thread's eight
+// entries are in flight together: 10M entries 254 us with five narrow gathers
+// and a search of the offsets per entry, 143 us so.
+__global__ void __launch_bounds__(kPackThreads, 4) k_pack_gather(
+    int64_t ne, int64_t ni, int64_t nt, const int64_t* __restrict__ offs, const uint32_t* __restrict__ img,
+    const uint32_t* __restrict__ feat, const uint32_t* __restrict__ ordinal, const ImageRow* __restrict__ rows,
+    const float* __restrict__ features, int wide_features, int wide_obs, const uint32_t* __restrict__ tile_base,
+    const uint32_t* __restrict__ tile_track, double* __restrict__ obs,
     uint32_t* __restrict__ camera_index, uint32_t* __restrict__ intrinsic_index, uint32_t* __restrict__ point_index,
     unsigned long long* __restrict__ counters) {
-  __shared__ uint32_t sh_warp[32];
+  __shared__ uint32_t sh_track[kPackTile];  // by entry: tracks past the tile's first that start at it (their last)
+  __shared__ uint32_t sh_cnt[kPackPer][kPackThreads / 32];
+  __shared__ uint32_t sh_max[kPackThreads / 32];
   unsigned long long err = 0;
-  uint32_t running = tile_base[blockIdx.x];
-  const int64_t tile = blockIdx.x * kPackTile;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t tile = blockIdx.x * kPackTile, end = min(ne, tile + kPackTile);
+  // the tracks that start in the tile: past that of its first entry, up to
+  // that of the next tile's first (on a valid CSR; a bad one only misplaces
+  // tracks of a call that fails)
+  const int64_t t0 = tile_track[blockIdx.x];
+  const int64_t t1 = end < ne ? min((int64_t)tile_track[blockIdx.x + 1], nt - 1) : nt - 1;
+  for (int i = tid; i < kPackTile; i += kPackThreads) sh_track[i] = 0;
+  // the entries (entry j * 256 + tid of the tile), all loads in flight
+  uint32_t im[kPackPer], f[kPackPer], ord[kPackPer];
+#pragma unroll
   for (int j = 0; j < kPackPer; ++j) {
-    const int64_t e = tile + j * kPackThreads + threadIdx.x;
-    uint32_t im = 0, total;
-    const bool flag = entry_kept(e, ne, ni, img, ordinal, &im);
-    const uint32_t pos = running + block_exclusive_count(flag, sh_warp, &total);
-    if (flag) {
-      const uint32_t f = feat[e];
-      const int64_t a = feature_offsets[im], b = feature_offsets[im + 1];
-      const bool ok = a >= 0 && b <= nf && (int64_t)f < b - a;
-      float x = 0.0f, y = 0.0f;
-      if (ok) {
-        x = features[2 * (a + f)];
-        y = features[2 * (a + f) + 1];
-      } else {
-        err |= kBadFeature;
-      }
-      int64_t lo = 0, hi = nt;  // offs[lo] <= e < offs[hi] on a valid CSR
-      while (hi - lo > 1) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (offs[mid] <= e) lo = mid; else hi = mid;
-      }
-      obs[2 * (int64_t)pos] = (double)x;
-      obs[2 * (int64_t)pos + 1] = (double)y;
-      camera_index[pos] = ordinal[im];
-      intrinsic_index[pos] = group[im];
-      point_index[pos] = (uint32_t)lo;
+    const int64_t e = tile + j * kPackThreads + tid;
+    im[j] = e < ne ? img[e] : 0xffffffffu;
+    f[j] = e < ne ? feat[e] : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < kPackPer; ++j) {
+    const int64_t e = tile + j * kPackThreads + tid;
+    ord[j] = e < ne && im[j] < (uint64_t)ni ? ordinal[im[j]] : kNoCamera;
+    const unsigned mask = __ballot_sync(0xffffffffu, ord[j] != kNoCamera);
+    if (lane == 0) sh_cnt[j][warp] = __popc(mask);
+  }
+  __syncthreads();
+  for (int64_t t = t0 + 1 + tid; t <= t1; t += kPackThreads) {
+    const int64_t o = offs[t] - tile;  // in (0, end - tile) on a valid CSR
+    if (o >= 0 && o < kPackTile) atomicMax(&sh_track[o], (uint32_t)(t - t0));
+  }
+  __syncthreads();
+  {
+    // running maximum: thread t over entries 8t .. 8t+7, then over the threads
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < kPackPer; ++k) m = max(m, sh_track[tid * kPackPer + k]);
+    uint32_t v = m;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v = max(v, u);
     }
-    running += total;
+    if (lane == 31) sh_max[warp] = v;
+    uint32_t run = __shfl_up_sync(0xffffffffu, v, 1);
+    if (lane == 0) run = 0;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) run = max(run, sh_max[w]);
+#pragma unroll
+    for (int k = 0; k < kPackPer; ++k) {
+      run = max(run, sh_track[tid * kPackPer + k]);
+      sh_track[tid * kPackPer + k] = run;
+    }
+  }
+  __syncthreads();
+  ImageRow row[kPackPer];
+#pragma unroll
+  for (int j = 0; j < kPackPer; ++j)
+    if (ord[j] != kNoCamera) row[j] = rows[im[j]];
+  float2 xy[kPackPer];
+#pragma unroll
+  for (int j = 0; j < kPackPer; ++j) {
+    xy[j] = make_float2(0.0f, 0.0f);
+    if (ord[j] == kNoCamera) continue;
+    const float* x = features + 2 * (row[j].first + f[j]);
+    if (f[j] >= row[j].count) err |= kBadFeature;
+    else if (wide_features) xy[j] = *reinterpret_cast<const float2*>(x);
+    else xy[j] = make_float2(x[0], x[1]);
+  }
+  uint32_t base = tile_base[blockIdx.x];
+#pragma unroll
+  for (int j = 0; j < kPackPer; ++j) {
+    uint32_t pos = base;
+#pragma unroll
+    for (int w = 0; w < kPackThreads / 32; ++w) {
+      const uint32_t c = sh_cnt[j][w];
+      if (w < warp) pos += c;
+      base += c;
+    }
+    const bool flag = ord[j] != kNoCamera;
+    pos += __popc(__ballot_sync(0xffffffffu, flag) & ((1u << lane) - 1u));
+    if (!flag) continue;
+    double* out = obs + 2 * (int64_t)pos;
+    if (wide_obs) {
+      *reinterpret_cast<double2*>(out) = make_double2((double)xy[j].x, (double)xy[j].y);
+    } else {
+      out[0] = (double)xy[j].x;
+      out[1] = (double)xy[j].y;
+    }
+    camera_index[pos] = ord[j];
+    intrinsic_index[pos] = row[j].group;
+    point_index[pos] = (uint32_t)(t0 + sh_track[j * kPackThreads + tid]);
   }
   if (err) atomicOr(&counters[2], err);
 }
@@ -803,9 +918,10 @@ gbba_status gbsfm_pack_ba(gbba_handle* h, const gbsfm_engine_state* st, int64_t 
     out->locked_camera = -1;
     const int64_t nb = std::max<int64_t>(1, ceil_div(ne, kPackTile));
     h->arena.reset();
-    h->arena.reserve(sizeof(gbsfm_camera) * ni + 16 * ni + sizeof(int64_t) * (ni + nt + 2) + sizeof(float) * 2 * nf +
+    const int64_t nchunks = ceil_div(std::max<int64_t>(1, ni), kImageChunk);
+    h->arena.reserve(sizeof(gbsfm_camera) * ni + (16 + sizeof(ImageRow)) * ni + 4 * nchunks + sizeof(int64_t) * (ni + nt + 2) + sizeof(float) * 2 * nf +
                      sizeof(uint32_t) * 2 * ne + sizeof(double) * 6 * ni + sizeof(double) * 2 * ne +
-                     sizeof(uint32_t) * 3 * ne + 4 * nb + 256 * 24);
+                     sizeof(uint32_t) * 3 * ne + 8 * nb + 256 * 24);
     const gbsfm_camera* dcam = in_view(h, st->cameras, ni, memory);
     const uint8_t* drec = in_view(h, st->reconstructed, ni, memory);
     const uint32_t* dgrp = in_view(h, st->intrinsic_group, ni, memory);
@@ -823,6 +939,9 @@ gbba_status gbsfm_pack_ba(gbba_handle* h, const gbsfm_engine_state* st, int64_t 
     uint32_t* dcimg = out_view(h, out->camera_image, ni, memory);
     uint32_t* ordinal = h->arena.take<uint32_t>(std::max<int64_t>(1, ni));
     uint32_t* tiles = h->arena.take<uint32_t>(nb);
+    uint32_t* tracks = h->arena.take<uint32_t>(nb);
+    uint32_t* chunks = h->arena.take<uint32_t>(nchunks);
+    ImageRow* rows = h->arena.take<ImageRow>(std::max<int64_t>(1, ni));
     unsigned long long* counters = h->arena.take<unsigned long long>(4);
     // intrinsic groups and points enter the problem as they are
     if (ng > 0 && out->intrinsics != st->group_intrinsics)
@@ -831,19 +950,28 @@ gbba_status gbsfm_pack_ba(gbba_handle* h, const gbsfm_engine_state* st, int64_t 
     if (nt > 0 && out->points != st->points)
       GBBA_CUDA(cudaMemcpyAsync(out->points, st->points, sizeof(double) * 3 * nt, cudaMemcpyDefault, h->active));
     GBBA_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), h->active));
+    GBBA_CUDA(cudaMemsetAsync(tracks, 0, sizeof(uint32_t) * nb, h->active));
     if (dcc && ni > 0) GBBA_CUDA(cudaMemsetAsync(dcc, 0, ni, h->active));
     KernelTimer timer(h);
     if (ni > 0) {
-      k_pack_images<<<1, 1024, 0, h->active>>>(ni, drec, dcam, dgrp, ng, ordinal, dext, dcimg, counters);
+      if (nchunks > 1) {
+        k_image_counts<<<(unsigned)nchunks, kImageThreads, 0, h->active>>>(ni, drec, chunks);
+        check_launch(h);
+      }
+      k_pack_images<<<(unsigned)ceil_div(ni, kImageThreads), kImageThreads, 0, h->active>>>(
+          ni, drec, dcam, dgrp, ng, chunks, dfo, nf, rows, ordinal, dext, dcimg, counters);
       check_launch(h);
     }
-    k_pack_count<<<(unsigned)nb, kPackThreads, 0, h->active>>>(ne, ni, nt, doff, dimg, ordinal, tiles, counters);
+    k_pack_count<<<(unsigned)nb, kPackThreads, 0, h->active>>>(ne, ni, nt, doff, dimg, ordinal, tiles, tracks,
+                                                            counters);
     check_launch(h);
     k_pack_scan<<<1, 1024, 0, h->active>>>(tiles, nb, counters);
     check_launch(h);
     if (ne > 0) {
-      k_pack_gather<<<(unsigned)nb, kPackThreads, 0, h->active>>>(ne, ni, nt, nf, doff, dimg, dfeat, ordinal, dgrp,
-                                                                  dfo, dft, tiles, dobs, dci, dii, dpi, counters);
+      auto aligned = [](const void* p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0 ? 1 : 0; };
+      k_pack_gather<<<(unsigned)nb, kPackThreads, 0, h->active>>>(ne, ni, nt, doff, dimg, dfeat, ordinal, rows, dft,
+                                                                  aligned(dft, 8), aligned(dobs, 16), tiles, tracks, dobs, dci,
+                                                                  dii, dpi, counters);
       check_launch(h);
     }
     if (ni > 0) {
