@@ -125,14 +125,45 @@ struct GlobalViews64 {
   }
 };
 
+// The block's tracks dealt to its threads in order of length (a counting sort,
+// longest first): the track number of this thread.  A warp takes as long as
+// its longest track.
+constexpr int kTriLens = 64;  // lengths told apart (longer tracks share the last)
+template <int kThreads, typename Off>
+__device__ __forceinline__ int64_t track_by_length(const Off* __restrict__ offs, int64_t t0, int64_t nt) {
+  __shared__ uint16_t order[kThreads];
+  __shared__ int len_count[kTriLens];
+  const int tl = threadIdx.x;
+  int len = 0;
+  if (t0 + tl < nt) {
+    const Off d = offs[t0 + tl + 1] - offs[t0 + tl];
+    len = d < (Off)kTriLens ? (int)d : kTriLens - 1;
+  }
+  for (int l = tl; l < kTriLens; l += kThreads) len_count[l] = 0;
+  __syncthreads();
+  const int rank = atomicAdd(&len_count[len], 1);  // any order among equal lengths: tracks are independent
+  __syncthreads();
+  int before = 0;
+  for (int l = len + 1; l < kTriLens; ++l) before += len_count[l];
+  order[before + rank] = (uint16_t)tl;
+  __syncthreads();
+  return t0 + order[tl];
+}
+
 // FP64 parity path, one thread per track: X [nt][4] (NVIEW / ALGEBRAIC) or
-// [nt][3] and Triangulation::error (ITERATIVE).
-__global__ void __launch_bounds__(128) k_nview64(int method, const double* __restrict__ P, const int64_t* __restrict__ offs,
+// [nt][3] and Triangulation::error (ITERATIVE).  Bound by FP64 operations:
+// 100,000 tracks of 2 to 30 views 1.9 ms, against 5.3 with Givens rotations,
+// three passes over the views and FP64 Jacobi sweeps for every track.
+constexpr int kNview64Threads = 128;
+__global__ void __launch_bounds__(kNview64Threads) k_nview64(int method, const double* __restrict__ P, const int64_t* __restrict__ offs,
                                                  const uint32_t* __restrict__ cam, const double* __restrict__ xy,
                                                  int64_t nt, double* __restrict__ X, double* __restrict__ err,
                                                  const unsigned int* __restrict__ bad) {
   if (*bad) return;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t t0 = blockIdx.x * (int64_t)kNview64Threads; t0 < nt; t0 += (int64_t)gridDim.x * kNview64Threads) {
+    __syncthreads();  // the order of the tracks before is no longer read
+    const int64_t t = track_by_length<kNview64Threads>(offs, t0, nt);
+    if (t >= nt) continue;
     const int64_t b = offs[t];
     const int n = (int)(offs[t + 1] - b);
     const GlobalViews64 views{P, cam, xy, b};
@@ -159,8 +190,11 @@ __global__ void __launch_bounds__(128) k_nview64(int method, const double* __res
       continue;
     }
     double Xh[4];
-    if (method == 0) nview_track<double>(views, n, Xh);
-    else algebraic_track<double>(views, n, Xh);
+    const bool done = method == 0 ? nview_track_short(views, n, Xh) : algebraic_track_short(views, n, Xh);
+    if (!done) {
+      if (method == 0) nview_track<double>(views, n, Xh);
+      else algebraic_track<double>(views, n, Xh);
+    }
 #pragma unroll
     for (int r = 0; r < 4; ++r) X[4 * t + r] = Xh[r];
   }
@@ -172,13 +206,11 @@ __global__ void __launch_bounds__(128) k_nview64(int method, const double* __res
 // (Triangulation::compute(3)); then gn_steps Gauss-Newton steps on the
 // reprojection error.
 //
-// A warp takes as long as its longest track, so a block's tracks are dealt to
-// its threads in order of length (a counting sort); blocks of 1,024 sort best
-// and, at 64 registers, hide the chains of square roots and divisions best:
+// A block's tracks are dealt to its threads by length; blocks of 1,024 sort
+// best and, at 64 registers, hide the chains of square roots and divisions best:
 // 1M tracks of 2 to 30 views 1.68 ms with 128 tracks in the caller's order,
 // 1.38 with 512, 1.23 with 1,024.  Batches that would leave SMs idle take
 // smaller blocks (launch below).
-constexpr int kTriLens = 64;     // lengths told apart by the sort (longer tracks share the last)
 constexpr int kTriCams = 1024;   // camera table kept in shared memory up to this size
 
 // A track's views: its observations straight from global memory (a track's are
@@ -210,20 +242,8 @@ __global__ void __launch_bounds__(kTriThreads, kBlocks) k_tri_f32(int method, co
   const int ncam_s = ncam <= kTriCams ? (int)ncam : 0;
   for (int i = threadIdx.x; i < ncam_s * 12; i += kTriThreads) sP[i] = P[i];
   const int64_t t0 = (int64_t)blockIdx.x * kTriThreads;
-  // tracks by length, longest first
-  __shared__ uint16_t order[kTriThreads];
-  __shared__ int len_count[kTriLens];
-  const int tl = threadIdx.x;
-  const int len = t0 + tl < nt ? (int)min(offs[t0 + tl + 1] - offs[t0 + tl], (uint32_t)(kTriLens - 1)) : 0;
-  for (int l = tl; l < kTriLens; l += kTriThreads) len_count[l] = 0;
   __syncthreads();
-  const int rank = atomicAdd(&len_count[len], 1);  // any order among equal lengths: tracks are independent
-  __syncthreads();
-  int before = 0;
-  for (int l = len + 1; l < kTriLens; ++l) before += len_count[l];
-  order[before + rank] = (uint16_t)tl;
-  __syncthreads();
-  const int64_t t = t0 + order[threadIdx.x];
+  const int64_t t = track_by_length<kTriThreads>(offs, t0, nt);
   if (t >= nt) return;
   const uint32_t b = offs[t], e = offs[t + 1];
   const int n = (int)(e - b);

@@ -347,6 +347,324 @@ __host__ __device__ void nview_track(const Views& view, int n, T X[4]) {
   nview_normalize<T>(Q, X);
 }
 
+// ---- the FP64 path's shorter way to the same vector.  FP64 operations bound
+// it on the GPU (two a clock per SM, and a square root or division is about ten),
+// so it spends fewer of them than nview_track:
+//   - the rows go into R two views at a time by Householder reflections (four
+//     square roots and divisions per two views instead of 16 and 32 of Givens
+//     rotations);
+//   - one pass over the views: G(lambda) and Q(lambda) from the moments
+//     G_m = sum h h^T / c^(2m), m = 1..4, whose next term is (lambda / c^2)^4
+//     smaller.  A track with lambda / c^2 above 5e-5 is left to nview_track;
+//   - the smallest singular pair of R L^-T by inverse iteration,
+//     X <- R^-1 R^-T G X, instead of Jacobi sweeps.
+// The sign of the vector is the one that the Jacobi sweeps give (they start
+// from the identity and each rotation is the smaller one): they run in FP32,
+// and a track whose rotations are not clear in FP32 (two columns of nearly
+// equal norm) is left to the FP64 sweeps.
+
+// Rotate four rows into the upper-triangular R (Householder).
+__host__ __device__ __forceinline__ void house_in4(double R[4][4], double rows[4][4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    double s2 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s2 += rows[i][k] * rows[i][k];
+    if (s2 == 0.0) continue;
+    const double a = R[k][k], nrm = sqrt(a * a + s2);
+    const double v0 = a >= 0.0 ? a + nrm : a - nrm;
+    const double tau = 1.0 / (nrm * fabs(v0));  // 2 / (v0^2 + s2)
+#pragma unroll
+    for (int l = k + 1; l < 4; ++l) {
+      double d = v0 * R[k][l];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d += rows[i][k] * rows[i][l];
+      d *= tau;
+      R[k][l] -= d * v0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) rows[i][l] -= d * rows[i][k];
+    }
+    R[k][k] = a >= 0.0 ? -nrm : nrm;
+  }
+}
+
+// min_right_singular4's vector in FP32; false when a rotation's direction or
+// the smallest column is within FP32 rounding of the other choice, or a value
+// is not finite.
+__host__ __device__ inline bool min_right_singular4_f32(float B[4][4], float y[4]) {
+  float V[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) V[i][j] = i == j ? 1.f : 0.f;
+  bool clear = true;
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    bool rotated = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = i + 1; j < 4; ++j) {
+        float a = 0.f, b = 0.f, g = 0.f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          a += B[r][i] * B[r][i];
+          b += B[r][j] * B[r][j];
+          g += B[r][i] * B[r][j];
+        }
+        clear = clear && fabsf(b - a) > 2e-5f * (a + b) && a + b < 1e30f;
+        if (fabsf(g) <= 1e-6f * sqrtf(a * b)) continue;
+        rotated = true;
+        const float zeta = (b - a) / (2.f * g);
+        const float t = (zeta >= 0.f ? 1.f : -1.f) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
+        const float cs = 1.f / sqrtf(1.f + t * t), sn = cs * t;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float ui = B[r][i], uj = B[r][j];
+          B[r][i] = cs * ui - sn * uj;
+          B[r][j] = sn * ui + cs * uj;
+          const float vi = V[r][i], vj = V[r][j];
+          V[r][i] = cs * vi - sn * vj;
+          V[r][j] = sn * vi + cs * vj;
+        }
+      }
+    if (!rotated) break;
+    if (sweep == 11) clear = false;
+  }
+  float n0 = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float nrm = B[0][i] * B[0][i] + B[1][i] * B[1][i] + B[2][i] * B[2][i] + B[3][i] * B[3][i];
+    clear = clear && nrm >= 0.f;  // not NaN
+    if (i == 0 || nrm < n0) {
+      n0 = nrm;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) y[r] = V[r][i];
+    }
+  }
+  return clear;
+}
+
+// X of the FP32 sweeps for R, G (G = L L^T, y the vector of R L^-T, X = L^-T y).
+__host__ __device__ inline bool nview_start_f32(const double R[4][4], const double G[10], double X[4]) {
+  float L[4][4], Li[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float d = (float)G[sym4(j, j)];
+#pragma unroll
+    for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
+    L[j][j] = sqrtf(d);
+#pragma unroll
+    for (int i = j + 1; i < 4; ++i) {
+      float v = (float)G[sym4(i, j)];
+#pragma unroll
+      for (int k = 0; k < j; ++k) v -= L[i][k] * L[j][k];
+      L[i][j] = v / L[j][j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    Li[j][j] = 1.f / L[j][j];
+#pragma unroll
+    for (int i = j + 1; i < 4; ++i) {
+      float v = 0.f;
+#pragma unroll
+      for (int k = j; k < i; ++k) v -= L[i][k] * Li[k][j];
+      Li[i][j] = v / L[i][i];
+    }
+  }
+  float B[4][4], y[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float v = 0.f;
+#pragma unroll
+      for (int k = i; k < 4; ++k)
+        if (k <= j) v += (float)R[i][k] * Li[j][k];
+      B[i][j] = v;
+    }
+  if (!min_right_singular4_f32(B, y)) return false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float v = 0.f;
+#pragma unroll
+    for (int j = i; j < 4; ++j) v += Li[j][i] * y[j];
+    X[i] = (double)v;
+  }
+  return true;
+}
+
+// Inverse iteration X <- R^-1 R^-T G X (scaled to unit norm) from X until it
+// moves by less than 1e-13 and once more; iR = 1 / diag(R).  *lam: the
+// Rayleigh quotient |R X|^2 / X^T G X.  False when 12 iterations do not get there.
+__host__ __device__ __forceinline__ bool nview_iterate(const double R[4][4], const double iR[4], const double G[10],
+                                                       double X[4], double* lam) {
+  bool last = false;
+  for (int it = 0; it < 12; ++it) {
+    double u[4], nn = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u[i] = 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[i] += G[sym4(i, j)] * X[j];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int k = 0; k < i; ++k) u[i] -= R[k][i] * u[k];
+      u[i] *= iR[i];
+    }
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+#pragma unroll
+      for (int k = i + 1; k < 4; ++k) u[i] -= R[i][k] * u[k];
+      u[i] *= iR[i];
+      nn += u[i] * u[i];
+    }
+    const double s = 1.0 / sqrt(nn);
+    double move = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const double x = u[i] * s;
+      move += (x - X[i]) * (x - X[i]);
+      X[i] = x;
+    }
+    if (last) {
+      double num = 0.0, den = 0.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        double r = 0.0, q = 0.0;
+#pragma unroll
+        for (int j = i; j < 4; ++j) r += R[i][j] * X[j];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q += G[sym4(i, j)] * X[j];
+        num += r * r;
+        den += X[i] * q;
+      }
+      *lam = num / den;
+      return true;
+    }
+    last = move < 1e-26;
+  }
+  return false;
+}
+
+// One pass over a track's views: R, and with kDepths the moments M[m] =
+// sum h h^T / c^(2m + 2) and the largest 1 / c^2 (TriangulateNView), else the
+// rows of the algebraic design.
+template <bool kDepths, typename Views>
+__host__ __device__ __forceinline__ void track_rows(const Views& view, int n, double R[4][4], double M[4][10],
+                                                    double* wmax) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) R[i][j] = 0.0;
+  if (kDepths) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int i = 0; i < 10; ++i) M[m][i] = 0.0;
+    *wmax = 0.0;
+  }
+  for (int j = 0; j < n; j += 2) {
+    double rows[4][4];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      if (j + v >= n) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rows[2 * v][k] = rows[2 * v + 1][k] = 0.0;
+        continue;
+      }
+      const double* P;
+      double px, py;
+      view(j + v, &P, &px, &py);
+      if (kDepths) {
+        double h[4], c;
+        view_house<double>(P, px, py, h, rows[2 * v], rows[2 * v + 1], &c);
+        double w = 1.0 / (c * c);
+        const double w1 = w;
+        *wmax = w > *wmax ? w : *wmax;
+        double hh[10];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = a; b < 4; ++b) hh[sym4(a, b)] = h[a] * h[b];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+#pragma unroll
+          for (int i = 0; i < 10; ++i) M[m][i] += w * hh[i];
+          w *= w1;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          rows[2 * v][k] = -P[4 + k] + py * P[8 + k];
+          rows[2 * v + 1][k] = P[k] - px * P[8 + k];
+        }
+      }
+    }
+    house_in4(R, rows);
+  }
+}
+
+// TriangulateNView of one track; false: the track is one for nview_track.
+template <typename Views>
+__host__ __device__ bool nview_track_short(const Views& view, int n, double X[4]) {
+  double R[4][4], M[4][10], wmax, iR[4];
+  track_rows<true>(view, n, R, M, &wmax);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    iR[i] = 1.0 / R[i][i];
+    if (!(fabs(iR[i]) < 1e150)) return false;
+  }
+  double lam = 0.0, Q[10];
+  for (int pass = 0; pass < 3; ++pass) {
+    double G[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) {
+      G[i] = M[0][i] + lam * (M[1][i] + lam * (M[2][i] + lam * M[3][i]));
+      Q[i] = M[0][i] + lam * (2.0 * M[1][i] + lam * (3.0 * M[2][i] + 4.0 * lam * M[3][i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) G[sym4(i, i)] += 1.0;
+    // the last pass's FP32 vector has the sign, the first one's starts the iteration
+    double S[4];
+    if (pass != 1) {
+      if (!nview_start_f32(R, G, S)) return false;
+      const double s = pass == 0 ? 1.0 : X[0] * S[0] + X[1] * S[1] + X[2] * S[2] + X[3] * S[3];
+      if (pass == 0) {
+        const double nn = 1.0 / sqrt(S[0] * S[0] + S[1] * S[1] + S[2] * S[2] + S[3] * S[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) X[i] = S[i] * nn;
+      } else if (s < 0.0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) X[i] = -X[i];
+      }
+    }
+    if (!nview_iterate(R, iR, G, X, &lam)) return false;
+    if (!(lam * wmax < 5e-5)) return false;
+  }
+  nview_normalize<double>(Q, X);
+  return true;
+}
+
+// TriangulateNViewAlgebraic of one track; false: the track is one for algebraic_track.
+template <typename Views>
+__host__ __device__ bool algebraic_track_short(const Views& view, int n, double X[4]) {
+  double R[4][4], iR[4], lam, S[4];
+  track_rows<false>(view, n, R, nullptr, nullptr);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    iR[i] = 1.0 / R[i][i];
+    if (!(fabs(iR[i]) < 1e150)) return false;
+  }
+  const double I[10] = {1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 1.0, 0.0, 1.0};
+  if (!nview_start_f32(R, I, S)) return false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) X[i] = S[i];
+  return nview_iterate(R, iR, I, X, &lam);
+}
+
 // TriangulateNViewAlgebraic of one track: unit X.
 template <typename T, typename Views>
 __host__ __device__ void algebraic_track(const Views& view, int n, T X[4]) {
