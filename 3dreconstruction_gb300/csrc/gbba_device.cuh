@@ -216,6 +216,74 @@ __device__ __forceinline__ void residual_pose(const T* __restrict__ Kp, const T*
   camera_residual<M, T, false>(Kp, p, ox, oy, r, Jk, D);
 }
 
+// Linearisation data of one camera (FP64), 22 values: R(w) row-major, t, the
+// left Jacobian J_l(w) of the rotation row-major (d(R X) = (J_l dw) x R X),
+// and 1 in the first-order branch of ceres's AngleAxisRotatePoint, whose
+// derivative is dw x X (J_l = I and X in the place of R X).
+//   J_l = a I + (1 - a) u u^T + b [u]x,  a = sin(th)/th,  b = (1 - cos(th))/th
+constexpr int kCamLin = 22;
+__device__ __forceinline__ void cam_lin(const double E[6], double* __restrict__ L) {
+  pose_matrix<double>(E, L);
+  const double th2 = E[0] * E[0] + E[1] * E[1] + E[2] * E[2];
+  double* J = L + 12;
+  if (th2 > DBL_EPSILON) {
+    const double th = sqrt(th2), ith = 1.0 / th;
+    double s, c, sh, ch;
+    sincos(th, &s, &c);
+    sincos(0.5 * th, &sh, &ch);
+    const double u[3] = {E[0] * ith, E[1] * ith, E[2] * ith};
+    const double a = s * ith, b = 2.0 * sh * sh * ith, d = 1.0 - a;
+    J[0] = a + d * u[0] * u[0];        J[1] = -b * u[2] + d * u[0] * u[1]; J[2] = b * u[1] + d * u[0] * u[2];
+    J[3] = b * u[2] + d * u[1] * u[0]; J[4] = a + d * u[1] * u[1];        J[5] = -b * u[0] + d * u[1] * u[2];
+    J[6] = -b * u[1] + d * u[2] * u[0]; J[7] = b * u[0] + d * u[2] * u[1]; J[8] = a + d * u[2] * u[2];
+    L[21] = 0.0;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) J[i] = i % 4 == 0 ? 1.0 : 0.0;
+    L[21] = 1.0;
+  }
+}
+
+// residual() with Jacobian blocks from a camera's linearisation data (16-byte
+// aligned): no sine, cosine or square root per observation, and
+//   dr/dw_k = D . (J_l e_k x q) = J_l e_k . (q x D),  q = R X
+// instead of the derivative of every Rodrigues term (about 130 FP64 operations
+// and a division against 400).
+template <int M>
+__device__ __forceinline__ void residual_lin(const double* __restrict__ Kp, const double* __restrict__ lin,
+                                             const double X[3], double ox, double oy, double r[2], double Je[2][6],
+                                             double Jk[2][Model<M>::K], double Jx[2][3]) {
+  double L[kCamLin];
+#pragma unroll
+  for (int i = 0; i < kCamLin; i += 2) {
+    const double2 v = __ldg(reinterpret_cast<const double2*>(lin + i));
+    L[i] = v.x;
+    L[i + 1] = v.y;
+  }
+  double p[3], q[3], D[2][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    q[i] = L[3 * i] * X[0] + L[3 * i + 1] * X[1] + L[3 * i + 2] * X[2];
+    p[i] = q[i] + L[9 + i];
+  }
+  if (L[21] != 0.0) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) q[i] = X[i];
+  }
+  camera_residual<M, double, true>(Kp, p, ox, oy, r, Jk, D);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double s[3] = {q[1] * D[i][2] - q[2] * D[i][1], q[2] * D[i][0] - q[0] * D[i][2],
+                         q[0] * D[i][1] - q[1] * D[i][0]};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      Je[i][k] = s[0] * L[12 + k] + s[1] * L[15 + k] + s[2] * L[18 + k];
+      Je[i][3 + k] = D[i][k];
+      Jx[i][k] = D[i][0] * L[k] + D[i][1] * L[3 + k] + D[i][2] * L[6 + k];
+    }
+  }
+}
+
 // Huber / squared loss: returns the cost 1/2 rho(s) and the Corrector scale sqrt(rho').
 template <typename T>
 __device__ __forceinline__ T robust(int loss_type, T a, T s, T* sqrt_rho1) {
@@ -259,6 +327,17 @@ __device__ __forceinline__ int lin_exp(unsigned long long mbits, double n) {
   frexp(m * n, &e);  // m n < 2^e
   return 62 - e;
 }
+// The same from an exponent e with |term| < 2^e for every term (above 1020:
+// non-finite; below every exponent: no term).
+__device__ __forceinline__ int lin_exp_of(int e, double n) {
+  if (e > 1020) return kFxNonFinite;
+  if (e < -4096) return 0;
+  int en;
+  frexp(n, &en);  // n < 2^en
+  return 62 - e - en;
+}
+// Exponent of a double, |v| < 2^e (no FP64 operation); above 1020 for infinities and NaN.
+__device__ __forceinline__ int exp_above(double v) { return (int)((__double2hiint(v) >> 20) & 0x7ff) - 1022; }
 // v 2^k rounded to an integer with integer operations (|v| 2^k < 2^62 by
 // the choice of k); any rounding rule serves, the sum is exact.
 __device__ __forceinline__ long long lin_fx(double v, int k) {
