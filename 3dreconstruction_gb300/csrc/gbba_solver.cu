@@ -157,6 +157,9 @@ struct Prob {
   // FP64 camera poses (pose_matrix, 12 per camera) of ext, or null: the
   // mixed path evaluates its FP64 residuals from them.
   const double* pose;
+  // FP64 linearisation data of the cameras (cam_lin), of ext: the FP64 path's
+  // Jacobian.
+  const double* lin;
   // FP32 copies of the parameters and of the Jacobi scales, or null: the
   // mixed path's FP32 Jacobian reads them instead of converting per
   // observation (conversions and FP64 products run on GB300's FP64 pipe).
@@ -180,8 +183,10 @@ struct ObsJac {
 };
 
 // Residual and Jacobian of observation o, robustified (Corrector) and, with
-// kScale, multiplied by the Jacobi column scaling.
-template <int M, typename T, bool kScale>
+// kScale, multiplied by the Jacobi column scaling.  kLin: the FP64 Jacobian
+// from the cameras' linearisation data (else from ext: the mixed path's FP64
+// point blocks).
+template <int M, typename T, bool kScale, bool kLin = sizeof(T) == 8>
 __device__ __forceinline__ void obs_jacobian(const Prob& P, int64_t o, const double* __restrict__ scale_c,
                                              const double* __restrict__ scale_p, ObsJac<M, T>& J, double* cost) {
   constexpr int K = Model<M>::K;
@@ -195,7 +200,13 @@ __device__ __forceinline__ void obs_jacobian(const Prob& P, int64_t o, const dou
   T Je[2][6], Jk[2][K], Jx[2][3];
   double r[2];
   double r_sr1 = -1.0;  // >= 0: r is already corrected and this is sqrt(rho') (residual cache)
-  if constexpr (sizeof(T) == 8) {
+  bool done = false;
+  if constexpr (sizeof(T) == 8 && kLin) {
+    done = P.lin != nullptr;
+    if (done) residual_lin<M>(Kd, P.lin + kCamLin * (int64_t)c, Xd, ob.x, ob.y, r, Je, Jk, Jx);
+  }
+  if (done) {
+  } else if constexpr (sizeof(T) == 8) {
     double Ed[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) Ed[i] = __ldg(&P.ext[6 * (int64_t)c + i]);
@@ -713,7 +724,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 1) k_schur_point_rec
         if (bad) {
           ObsJac<M, double> J64;
           double c64, g64[3];
-          obs_jacobian<M, double, true>(P, o, scale_c, scale_p, J64, &c64);
+          obs_jacobian<M, double, true, false>(P, o, scale_c, scale_p, J64, &c64);
           point_terms<M, double>(J64, v64, g64);
         }
 #pragma unroll
@@ -2562,6 +2573,20 @@ __global__ void k_cam_pose(const double* __restrict__ ext, int64_t nc, double* _
   for (int i = 0; i < 12; ++i) pose[12 * c + i] = q[i];
 }
 
+// FP64 linearisation data of ext (one thread per camera).
+// With it an FP64 Jacobian takes no rotation terms of its own: 300 cameras, 600k
+// observations, 5 iterations 98.5 -> 93.9 ms, 200 cameras, 400k: 42.0 -> 37.0 ms.
+__global__ void __launch_bounds__(64) k_cam_lin(const double* __restrict__ ext, int64_t nc, double* __restrict__ lin) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= nc) return;
+  double E[6], L[kCamLin];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) E[i] = ext[6 * c + i];
+  cam_lin(E, L);
+#pragma unroll
+  for (int i = 0; i < kCamLin; ++i) lin[kCamLin * c + i] = L[i];
+}
+
 // FP64 robustified cost 1/2 sum rho(|r|^2) at (ext, intr, pts); per-block partials.
 template <int M>
 __global__ void __launch_bounds__(256) k_cost(Prob P, const double* ext, const double* intr, const double* pts,
@@ -2659,7 +2684,8 @@ struct Solve {
   int precision;
   // device arrays
   double *ext, *intr, *pts, *ext2, *intr2, *pts2;
-  double *pose = nullptr, *pose2 = nullptr;  // FP64 poses of ext / ext2 (mixed path)
+  double *pose = nullptr, *pose2 = nullptr;  // FP64 poses of ext (mixed path) / ext2
+  double* lin = nullptr;                     // FP64 path: linearisation data of ext
   float *ext_f = nullptr, *intr_f = nullptr, *pts_f = nullptr;  // FP32 copies of ext, intr, pts (mixed path)
   float4* rcache = nullptr;  // mixed path: residual cache, [2][no] (current parameters, candidate)
   float* pcg_yf = nullptr;  // mixed path: FP32 point temporaries of the implicit product
@@ -2724,7 +2750,7 @@ static Prob make_prob(const Solve& s, const double* ext, const double* intr, con
   P.no = s.no;
   P.loss_type = o ? o->loss_type : 0;
   P.loss_a = o ? o->loss_scale : 1.0;
-  P.pose = nullptr;
+  P.pose = P.lin = nullptr;
   P.ext_f = P.intr_f = P.pts_f = P.scale_cf = P.scale_pf = nullptr;
   P.rc = nullptr;
   P.rc_out = nullptr;
@@ -2740,6 +2766,7 @@ static void carve(A& a, Solve& s, size_t tsize) {
   s.ext2 = a.template take<double>(6 * s.nc);
   s.pose = a.template take<double>(12 * s.nc);
   s.pose2 = a.template take<double>(12 * s.nc);
+  s.lin = a.template take<double>(tsize == 8 ? kCamLin * s.nc : 0);
   s.ext_f = a.template take<float>(6 * s.nc);
   s.intr_f = a.template take<float>((int64_t)s.k * s.ni);
   s.pts_f = a.template take<float>(3 * s.np);
@@ -3298,6 +3325,18 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   // s.pose for the current parameters, s.pose2 for the evaluated ones.
   constexpr bool kPose = sizeof(T) == 4;
   const unsigned nb_cam_pose = (unsigned)std::max<int64_t>(1, ceil_div(s.nc, 128));
+  // The FP64 path shares per-camera terms from 16384 observations on, where a
+  // launch for them (5 us) costs less than the Rodrigues terms of every
+  // observation (about 90 FP64 operations a cost, 300 a Jacobian); at 800
+  // observations both ways measured the same.
+  const bool many = !kPose && s.no >= 16384;
+  // camera data of the current parameters: poses (mixed path) or linearisation data (FP64 path)
+  auto camera_data = [&]() {
+    if (s.nc == 0) return;
+    if (kPose) k_cam_pose<<<nb_cam_pose, 128, 0, st>>>(s.ext, s.nc, s.pose);
+    else if (many) k_cam_lin<<<(unsigned)ceil_div(s.nc, 64), 64, 0, st>>>(s.ext, s.nc, s.lin);
+    check_launch(h);
+  };
   auto to_float = [&](const double* src, float* dst, int64_t n) {
     if (n <= 0) return;
     k_convert<double, float><<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 1024), 256, 0, st>>>(src, dst, n);
@@ -3308,7 +3347,7 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
     // the mixed path's residual cache: current parameters in slot 0, the
     // candidate in slot 1 (copied to slot 0 when the step is accepted)
     if (kPose && s.rcache) Pc.rc_out = s.rcache + (e == s.ext ? 0 : s.no);
-    if (kPose && s.nc > 0) {
+    if ((kPose || many) && s.nc > 0) {
       k_cam_pose<<<nb_cam_pose, 128, 0, st>>>(e, s.nc, s.pose2);
       check_launch(h);
       Pc.pose = s.pose2;
@@ -3319,11 +3358,9 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   // gradient max norm and x norm at the current point; scale on first use
   auto linearize = [&](bool first, double* gmax, double* xnorm) {
     Prob P = make_prob(s, s.ext, s.intr, s.pts, o);
-    if (kPose && s.nc > 0) {
-      k_cam_pose<<<nb_cam_pose, 128, 0, st>>>(s.ext, s.nc, s.pose);
-      check_launch(h);
-      P.pose = s.pose;
-    }
+    camera_data();
+    if (kPose) P.pose = s.pose;
+    else if (many) P.lin = s.lin;
     if (kPose) {
       to_float(s.ext, s.ext_f, 6 * s.nc);
       to_float(s.intr, s.intr_f, (int64_t)s.k * s.ni);
@@ -3394,10 +3431,7 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   // (k_schur_point_rec, k_rhs_camera), so no separate Jacobian pass runs.
   const bool fused = s.pair_path;
   auto refresh = [&]() {
-    if (kPose && s.nc > 0) {
-      k_cam_pose<<<nb_cam_pose, 128, 0, st>>>(s.ext, s.nc, s.pose);
-      check_launch(h);
-    }
+    camera_data();
     if (kPose) {
       to_float(s.ext, s.ext_f, 6 * s.nc);
       to_float(s.intr, s.intr_f, (int64_t)s.k * s.ni);
@@ -3461,7 +3495,9 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   // copied back), so the sequence is invariant and is captured once into CUDA
   // graphs that every iteration replays.
   Prob P = make_prob(s, s.ext, s.intr, s.pts, o);
-  if (kPose && s.nc > 0) P.pose = s.pose;  // refreshed by linearize() after every accepted step
+  // refreshed by linearize() or refresh() after every accepted step
+  if (kPose) P.pose = s.pose;
+  else if (many) P.lin = s.lin;
   // gradient norm of the fused linearisation: only with a gradient tolerance
   unsigned long long* const gshards = o->gradient_tolerance > 0.0 ? s.gmax_shards : nullptr;
   if (kPose) {
@@ -3503,20 +3539,24 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
                   P, s.pt_grp, s.n_pgrp, s.scale_c, s.scale_p, s.diag_p, o->min_lm_diagonal, o->max_lm_diagonal,
                   gshards, s.radius, (T*)s.Vinv, (T*)s.gpv, (T*)s.rec, s.flag);
           };
-          if (kPose && (o->mixed_flags & GBBA_MIXED_FP64_POINT_INVERSE))
-            point_rec(std::true_type());
-          else
-            point_rec(std::false_type());
+          bool fp64_inverse = false, kahan = false;  // the mixed path's safeguards
+          if constexpr (kPose) {
+            fp64_inverse = o->mixed_flags & GBBA_MIXED_FP64_POINT_INVERSE;
+            kahan = o->mixed_flags & GBBA_MIXED_KAHAN_SCHUR;
+            if (fp64_inverse) point_rec(std::true_type());
+          }
+          if (!fp64_inverse) point_rec(std::false_type());
           check_launch(h);
           if (s.dense && s.n_blocks > 0) {
-            if (kPose && (o->mixed_flags & GBBA_MIXED_KAHAN_SCHUR))
-              k_schur_pairs<B, T, true><<<(unsigned)ceil_div(s.n_blocks * 32, 128), 128, 0, st>>>(
+            auto pairs = [&](auto k) {
+              k_schur_pairs<B, T, decltype(k)::value><<<(unsigned)ceil_div(s.n_blocks * 32, 128), 128, 0, st>>>(
                   (const PairItem*)s.pair_items, s.n_blocks, s.pairs, (const T*)s.rec, s.ext_col, s.intr_col,
                   s.cam_group, s.k, s.nc, S, s.n_pad, (T*)s.pair_partial);
-            else
-              k_schur_pairs<B, T><<<(unsigned)ceil_div(s.n_blocks * 32, 128), 128, 0, st>>>(
-                  (const PairItem*)s.pair_items, s.n_blocks, s.pairs, (const T*)s.rec, s.ext_col, s.intr_col,
-                  s.cam_group, s.k, s.nc, S, s.n_pad, (T*)s.pair_partial);
+            };
+            if constexpr (kPose) {
+              if (kahan) pairs(std::true_type());
+            }
+            if (!kahan) pairs(std::false_type());
             check_launch(h);
             if (s.n_merges > 0) {
               k_pair_merge<B, T><<<(unsigned)ceil_div(s.n_merges * 32, 128), 128, 0, st>>>(

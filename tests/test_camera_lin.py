@@ -64,3 +64,22 @@ def test_gradient_routes_agree(model, mixed, handle, abi, scenes):
     handle.check(fn(handle.h, C.byref(p), abi.LOSS_HUBER, 4.0, None, None, None, g.ctypes.data), "backward")
     np.testing.assert_array_equal(g, full)
     assert (full[-9:] == 0).all() and np.isfinite(full).all()
+
+
+@pytest.mark.parametrize("cut", [1, 0, -1])
+def test_solver_on_both_sides_of_the_rule(cut, handle, abi, scenes, oracle_mod):
+    """16383, 16384 and 16385 observations (the solver takes the linearisation
+    data from 16384 on) against the oracle's iterations, with the tolerances
+    of the other FP64 comparisons."""
+    sc = scenes.medium_scene(num_cameras=12, num_points=4000, mean_views=5, seed=71, hold=(0, 1))
+    assert len(sc["observations"]) >= 16385
+    for k in ("observations", "camera_index", "intrinsic_index", "point_index"):
+        sc[k] = sc[k][:16384 - cut]
+    opts = scenes.ba_options_for(sc, max_num_iterations=2)
+    hp = abi.HostProblem(sc)
+    s = handle.solve(hp, opts)
+    _, so, po, _ = oracle_mod.ba_solve(sc, opts)
+    assert s.usable and s.num_iterations == so["num_iterations"]
+    assert abs(s.final_cost - so["final_cost"]) <= 1e-9 * so["final_cost"]
+    np.testing.assert_allclose(hp.extrinsics.reshape(-1, 6), np.asarray(po["extrinsics"]).reshape(-1, 6), rtol=0,
+                               atol=1e-8)
