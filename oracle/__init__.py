@@ -19,9 +19,10 @@ _lib = None
 
 def reference_dir():
     """Root of the reference's sources, from GBBA_REFERENCE_DIR (the same
-    variable the oracle Makefile reads), or None when they are not present."""
+    variable the oracle Makefile reads), or None when they are not present
+    (no directory, or an empty one)."""
     d = os.environ.get("GBBA_REFERENCE_DIR") or _default_reference_dir()
-    return d if os.path.isdir(d) else None
+    return d if os.path.isdir(d) and os.listdir(d) else None
 
 
 def _default_reference_dir():
