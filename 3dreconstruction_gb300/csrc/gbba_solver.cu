@@ -526,9 +526,10 @@ __global__ void __launch_bounds__(128) k_schur_point(Prob P, const double* __res
 }
 
 // ---------------------------------------------------------------- atomic-free Schur build
-// Used when every free intrinsic block belongs to a single camera (per-camera
-// intrinsics, or intrinsics held): the camera-side columns of an observation
-// are then owned by its camera, so S splits into camera-pair blocks.
+// Used when every camera has one intrinsic group.  With per-camera or held
+// intrinsics the camera-side columns of an observation are owned by its camera,
+// and S splits into camera-pair blocks; with free groups of several cameras it
+// does for the extrinsics, and the intrinsic rows come from k_group_*.
 //
 // Per-observation record of 9B + 8 values (B = 6 + K):
 //   [ Jc (2 x B) | W = Jc^T Jp (B x 3) | W V^-1 (B x 3) | q = Jc^T r - W V^-1 g_p (B) | Jp (2 x 3) | r (2) ]
@@ -1098,8 +1099,8 @@ template <int B>
 struct PairTile {
   static constexpr int TPD = (B + 2) / 3;
   static constexpr int NT = TPD * TPD;
-  static constexpr int G = NT <= 16 ? 2 : 1;
-  static constexpr int LPG = NT <= 16 ? 16 : 32;
+  static constexpr int G = NT <= 4 ? 8 : NT <= 16 ? 2 : 1;
+  static constexpr int LPG = 32 / G;
   static constexpr int WSZ = TPD * 12;
   static constexpr int JSZ = 2 * TPD * 4;
   static constexpr int PSZ = 2 * WSZ + JSZ;
@@ -1113,7 +1114,13 @@ __device__ __forceinline__ void lds12(const T* p, T v[12]) {
   for (int q = 0; q < 3; ++q) ld4<T>(p + 4 * q, v + 4 * q);
 }
 
-template <int B, typename T, bool kKahan = false>
+// BB: rows and columns of the block that are formed, the first BB of B (the
+// intrinsics' are left out where no camera owns them: a quarter of the
+// products, and 8 pairs at a time instead of 2).
+// FP64: bound by its pipe (a block of 12 takes 432 multiply-adds a pair; 2.2M
+// pairs 3.0 -> 2.2 ms with three instructions a product instead of four, floor
+// 1.6); 3.3M pairs of 6 rows 1.26 ms.
+template <int B, typename T, bool kKahan = false, int BB = B>
 __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict__ items, int64_t nitems,
                                                      const unsigned long long* __restrict__ pairs,
                                                      const T* __restrict__ rec, const int32_t* __restrict__ ext_col,
@@ -1121,12 +1128,13 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
                                                      const int32_t* __restrict__ cam_group, int K, int64_t nc,
                                                      T* __restrict__ S, int64_t ld, T* __restrict__ partial) {
   using R = Rec<B>;
-  using PT = PairTile<B>;
+  using PT = PairTile<BB>;
   // Pairs per stage: small stages keep registers and shared memory low, so
   // that many warps have loads in flight (measured on the medium workload,
   // 2 pairs per stage beat 4, 8 and 16).
-  constexpr int ST = 2;
-  __shared__ __align__(16) T sh[4][ST * PT::PSZ];
+  constexpr int ST = PT::G > 2 ? PT::G : 2;
+  constexpr int PSZ = PT::PSZ + (PT::G == 8 ? 16 / (int)sizeof(T) : 0);  // 8 groups: odd in 16 bytes, no bank conflicts
+  __shared__ __align__(16) T sh[4][ST * PSZ];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (w >= nitems) return;
@@ -1137,20 +1145,20 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
 #pragma unroll
   for (int u = 0; u < PT::SLOTS; ++u) {
     const int f = lane + 32 * u;
-    if (f < 3 * B) {
+    if (f < 3 * BB) {
       const int i = f / 3, k = f % 3;
       kind[u] = 0;
       src[u] = R::kWh + f;
       dst[u] = (i / 3) * 12 + (i % 3) * 3 + k;
-    } else if (f < 6 * B) {
-      const int g = f - 3 * B, i = g / 3, k = g % 3;
+    } else if (f < 6 * BB) {
+      const int g = f - 3 * BB, i = g / 3, k = g % 3;
       kind[u] = 1;
       src[u] = R::kW + g;
       dst[u] = PT::WSZ + (i / 3) * 12 + (i % 3) * 3 + k;
-    } else if (f < 8 * B) {
-      const int g = f - 6 * B, r = g / B, i = g % B;
+    } else if (f < 8 * BB) {
+      const int g = f - 6 * BB, r = g / BB, i = g % BB;
       kind[u] = 2;
-      src[u] = R::kJc + g;
+      src[u] = R::kJc + r * B + i;
       dst[u] = 2 * PT::WSZ + r * PT::TPD * 4 + (i / 3) * 4 + i % 3;
     } else {
       kind[u] = 3;
@@ -1217,7 +1225,7 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
       if (q < n) {
 #pragma unroll
         for (int u = 0; u < PT::SLOTS; ++u)
-          if (kind[u] != 3) sw[q * PT::PSZ + dst[u]] = v[q][u];
+          if (kind[u] != 3) sw[q * PSZ + dst[u]] = v[q][u];
       }
   };
   if (it.begin < it.end) stage_load(it.begin);
@@ -1238,7 +1246,7 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
     }
     if (active) {
       for (int q = grp; q < n; q += PT::G) {
-        const T* sp = sw + q * PT::PSZ;
+        const T* sp = sw + q * PSZ;
         T A[12], Bv[12];
         lds12<T>(sp + ti * 12, A);
         lds12<T>(sp + PT::WSZ + tj * 12, Bv);
@@ -1246,7 +1254,11 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
         for (int r = 0; r < 3; ++r)
 #pragma unroll
           for (int c = 0; c < 3; ++c)
-            add(r, c, -(A[3 * r] * Bv[3 * c] + A[3 * r + 1] * Bv[3 * c + 1] + A[3 * r + 2] * Bv[3 * c + 2]));
+            if constexpr (sizeof(T) == 8)  // three operations of the FP64 pipe instead of four
+              acc[r][c] = fma(-A[3 * r + 2], Bv[3 * c + 2],
+                              fma(-A[3 * r + 1], Bv[3 * c + 1], fma(-A[3 * r], Bv[3 * c], acc[r][c])));
+            else
+              add(r, c, -(A[3 * r] * Bv[3 * c] + A[3 * r + 1] * Bv[3 * c + 1] + A[3 * r + 2] * Bv[3 * c + 2]));
         if (same_bits & (1u << q)) {
           T ja0[4], ja1[4], jb0[4], jb1[4];
           ld4<T>(sp + 2 * PT::WSZ + ti * 4, ja0);
@@ -1267,25 +1279,26 @@ __global__ void __launch_bounds__(128) k_schur_pairs(const PairItem* __restrict_
 #pragma unroll
       for (int c = 0; c < 3; ++c) acc[r][c] -= cmp[r][c];
   }
-  if (PT::G == 2) {
+#pragma unroll
+  for (int d = 16; d >= PT::LPG && PT::G > 1; d >>= 1) {
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[r][c] += __shfl_down_sync(0xffffffffu, acc[r][c], 16);
+      for (int c = 0; c < 3; ++c) acc[r][c] += __shfl_down_sync(0xffffffffu, acc[r][c], d);
   }
   if (!active || grp != 0) return;
   const uint32_t ca = (uint32_t)(it.key / nc), cb = (uint32_t)(it.key % nc);
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     const int i = 3 * ti + r;
-    if (i >= B) continue;
+    if (i >= BB) continue;
     const int ci = it.slot >= 0 ? 0 : cam_col(ext_col, intr_col, cam_group, K, ca, i);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int j = 3 * tj + c;
-      if (j >= B) continue;
+      if (j >= BB) continue;
       if (it.slot >= 0) {
-        partial[(int64_t)it.slot * B * B + i * B + j] = acc[r][c];
+        partial[(int64_t)it.slot * BB * BB + i * BB + j] = acc[r][c];
         continue;
       }
       const int cj = cam_col(ext_col, intr_col, cam_group, K, cb, j);
@@ -1479,6 +1492,227 @@ __global__ void __launch_bounds__(kRhsThreads) k_rhs_camera(const uint32_t* __re
         atomicMax(gmax_shards + (c & (kGmaxShards - 1)),
                   (unsigned long long)__double_as_longlong(fabs(g / scale_c[ci])));
     }
+  }
+}
+
+// ---------------------------------------------------------------- shared intrinsics
+// Free intrinsic groups that several cameras use (one body for many images).
+// The camera-pair blocks then cover the extrinsics alone, and the rows of a
+// group g have a writer of their own, from sums over the points:
+//   G_pg = sum of the intrinsic rows of W over point p's observations of g
+//   H_pg = G_pg V_p^-1
+//   S[g][c]  = sum_o Jk_o^T Je_o [c uses g] - H_p(o)g W_e,o^T   (o of camera c)
+//   S[g][g'] = sum_o Jk_o^T Jk_o [g = g']   - sum_p H_pg G_pg'^T
+// so a point costs views x groups small products instead of the views^2
+// intrinsic rows of its camera pairs, and nothing is added with atomics.  300
+// cameras, 600k observations, 3 groups: 2.1 ms for the blocks and groups of an
+// iteration where the point-major build takes 10.1 (and 3.3 more for its
+// linearisation, 2.7 for its back substitution).  What is left is the FP64
+// pipe: 0.36 G multiply-adds in the pair blocks, 0.24 G in k_group_camera
+// (610 us; floor 420).
+
+// G, H (K x 3 each per point and group, [np][ng]) and the groups of each point
+// as a bit mask: one thread per row, a point's rows side by side.
+template <int B, typename T>
+__global__ void __launch_bounds__(256) k_group_points(const uint32_t* __restrict__ pt_off,
+                                                      const uint32_t* __restrict__ icam,
+                                                      const int32_t* __restrict__ group_idx, int64_t np, int ng,
+                                                      const T* __restrict__ rec, const T* __restrict__ Vinv,
+                                                      T* __restrict__ G, T* __restrict__ H,
+                                                      unsigned long long* __restrict__ mask) {
+  constexpr int K = B - 6;
+  using R = Rec<B>;
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= np * ng * K) return;
+  const int i = (int)(e % K);
+  const int64_t pg = e / K, p = pg / ng;
+  const int g = (int)(pg - p * ng);
+  T w[3] = {T(0), T(0), T(0)};
+  unsigned long long m = 0;
+  for (uint32_t o = pt_off[p]; o < pt_off[p + 1]; ++o) {
+    const int gi = group_idx[icam[o]];
+    if (gi >= 0) m |= 1ull << gi;
+    if (gi != g) continue;
+    const T* r = rec + (int64_t)o * R::kSize + R::kW + 3 * (6 + i);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) w[j] += r[j];
+  }
+  const T* v = Vinv + 6 * p;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) G[3 * e + j] = w[j];
+  H[3 * e] = w[0] * v[0] + w[1] * v[1] + w[2] * v[2];
+  H[3 * e + 1] = w[0] * v[1] + w[1] * v[3] + w[2] * v[4];
+  H[3 * e + 2] = w[0] * v[2] + w[1] * v[4] + w[2] * v[5];
+  if (g == 0 && i == 0) mask[p] = m;
+}
+
+// One block per camera c and y: y < ng writes S[group y][extrinsics of c]; y =
+// ng leaves the camera's share of its own group in camp[c][K][K + 2], Jk^T Jk
+// | q | Jk^T r.  A warp takes 32 / 6 (or 32 / K) observations at a time, a lane
+// per row: few sums a lane, so that many warps are in flight, and the rows of
+// an observation read together.  Sums in a fixed order.
+constexpr int kGroupThreads = 256;
+template <int B, typename T>
+__global__ void __launch_bounds__(kGroupThreads) k_group_camera(
+    const uint32_t* __restrict__ cam_off, const uint32_t* __restrict__ cam_obs, const uint32_t* __restrict__ pt,
+    const int32_t* __restrict__ cam_group, const int32_t* __restrict__ group_idx, const int32_t* __restrict__ groups,
+    int ng, const T* __restrict__ rec, const T* __restrict__ H, const unsigned long long* __restrict__ mask,
+    const int32_t* __restrict__ ext_col, const int32_t* __restrict__ intr_col, T* __restrict__ S, int64_t ld,
+    double* __restrict__ camp) {
+  constexpr int K = B - 6, W = kGroupThreads / 32;
+  constexpr int SE = 32 / 6, SK = 32 / K;
+  constexpr int kPart = W * SE * 6 * K > W * SK * K * (K + 2) ? W * SE * 6 * K : W * SK * K * (K + 2);
+  using R = Rec<B>;
+  __shared__ T part[kPart];
+  const int64_t c = blockIdx.x;
+  const int y = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t q0 = cam_off[c], q1 = cam_off[c + 1];
+  if (q0 == q1) return;
+  const int own = group_idx[cam_group[c]];
+  if (y < ng) {
+    const int i = lane % 6, slot = lane / 6;
+    if (slot < SE) {
+      T acc[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) acc[k] = T(0);
+      for (uint32_t q = q0 + warp * SE + slot; q < q1; q += W * SE) {
+        const uint32_t o = cam_obs[q], p = pt[o];
+        if (!((mask[p] >> y) & 1)) continue;
+        const T* r = rec + (int64_t)o * R::kSize;
+        const T* h = H + ((int64_t)p * ng + y) * (3 * K);
+        const T w0 = r[R::kW + 3 * i], w1 = r[R::kW + 3 * i + 1], w2 = r[R::kW + 3 * i + 2];
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] = fma(-w2, h[3 * k + 2], fma(-w1, h[3 * k + 1], fma(-w0, h[3 * k], acc[k])));
+        if (y == own) {
+          const T e0 = r[R::kJc + i], e1 = r[R::kJc + B + i];
+#pragma unroll
+          for (int k = 0; k < K; ++k) acc[k] = fma(e1, r[R::kJc + B + 6 + k], fma(e0, r[R::kJc + 6 + k], acc[k]));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) part[((warp * SE + slot) * 6 + i) * K + k] = acc[k];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 6 * K; e += kGroupThreads) {
+      double v = 0.0;
+      for (int w = 0; w < W * SE; ++w) v += (double)part[w * 6 * K + e];
+      const int cj = ext_col[6 * c + e / K], ci = intr_col[(int64_t)K * groups[y] + e % K];
+      if (ci >= 0 && cj >= 0) S[(int64_t)ci * ld + cj] = (T)v;  // intrinsic columns come after the extrinsic ones
+    }
+    return;
+  }
+  if (own < 0) return;
+  const int i = lane % K, slot = lane / K;
+  if (slot < SK) {
+    T acc[K + 2];
+#pragma unroll
+    for (int k = 0; k < K + 2; ++k) acc[k] = T(0);
+    for (uint32_t q = q0 + warp * SK + slot; q < q1; q += W * SK) {
+      const T* r = rec + (int64_t)cam_obs[q] * R::kSize;
+      const T j0 = r[R::kJc + 6 + i], j1 = r[R::kJc + B + 6 + i];
+#pragma unroll
+      for (int k = 0; k < K; ++k) acc[k] = fma(j1, r[R::kJc + B + 6 + k], fma(j0, r[R::kJc + 6 + k], acc[k]));
+      acc[K] += r[R::kQ + 6 + i];
+      acc[K + 1] = fma(j1, r[R::kR + 1], fma(j0, r[R::kR], acc[K + 1]));
+    }
+#pragma unroll
+    for (int k = 0; k < K + 2; ++k) part[((warp * SK + slot) * K + i) * (K + 2) + k] = acc[k];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < K * (K + 2); e += kGroupThreads) {
+    double v = 0.0;
+    for (int w = 0; w < W * SK; ++w) v += (double)part[w * K * (K + 2) + e];
+    camp[c * K * (K + 2) + e] = v;
+  }
+}
+
+// Groups (g, g') of pair number y, g >= g'.
+__device__ __forceinline__ int2 group_pair(int y) {
+  int g = 0;
+  while ((g + 1) * (g + 2) / 2 <= y) ++g;
+  return make_int2(g, y - g * (g + 1) / 2);
+}
+
+// sum over the points of H_pg G_pg'^T: block x of pair y leaves one partial sum.
+template <int K, typename T>
+__global__ void __launch_bounds__(kGroupThreads) k_group_pairs(int64_t np, int ng, const T* __restrict__ G,
+                                                               const T* __restrict__ H,
+                                                               const unsigned long long* __restrict__ mask,
+                                                               double* __restrict__ partial) {
+  constexpr int W = kGroupThreads / 32, SK = 32 / K;
+  __shared__ T part[W * SK * K * K];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = lane % K, slot = lane / K;
+  const int2 gg = group_pair(blockIdx.y);
+  if (slot < SK) {
+    T acc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = T(0);
+    for (int64_t p = (blockIdx.x * (int64_t)W + warp) * SK + slot; p < np; p += (int64_t)gridDim.x * W * SK) {
+      const unsigned long long m = mask[p];
+      if (!((m >> gg.x) & (m >> gg.y) & 1)) continue;
+      const T* h = H + ((p * ng + gg.x) * K + i) * 3;
+      const T* g = G + (p * ng + gg.y) * (3 * K);
+#pragma unroll
+      for (int k = 0; k < K; ++k) acc[k] = fma(h[2], g[3 * k + 2], fma(h[1], g[3 * k + 1], fma(h[0], g[3 * k], acc[k])));
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) part[((warp * SK + slot) * K + i) * K + k] = acc[k];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < K * K; e += kGroupThreads) {
+    double v = 0.0;
+    for (int w = 0; w < W * SK; ++w) v += (double)part[w * K * K + e];
+    partial[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * K * K + e] = v;
+  }
+}
+
+// S[g][g'] of one pair of groups from the partial sums, and for g = g' the
+// group's rhs, LM diagonal and gradient norm (as k_rhs_camera's).
+template <int K, typename T>
+__global__ void __launch_bounds__(kGroupThreads) k_group_merge(
+    int64_t nc, const int32_t* __restrict__ cam_group, const int32_t* __restrict__ group_idx,
+    const int32_t* __restrict__ groups, const double* __restrict__ camp, const double* __restrict__ partial, int nb,
+    const int32_t* __restrict__ intr_col, T* __restrict__ S, int64_t ld, T* __restrict__ rhs,
+    const double* __restrict__ scale_c, double* __restrict__ diag_c, double dmin, double dmax,
+    const double* __restrict__ radius, unsigned long long* __restrict__ gmax_shards) {
+  constexpr int E = K * (K + 2), NS = kGroupThreads / E;
+  __shared__ double part[2][NS * E];
+  const int2 gg = group_pair(blockIdx.x);
+  const int e = threadIdx.x % E, sl = threadIdx.x / E, i = e / (K + 2), k = e % (K + 2);
+  double u = 0.0, w = 0.0;
+  if (sl < NS) {
+    if (k < K)
+      for (int x = sl; x < nb; x += NS) w += partial[((int64_t)blockIdx.x * nb + x) * K * K + i * K + k];
+    if (gg.x == gg.y) {
+      for (int64_t c = sl; c < nc; c += NS)
+        if (cam_group[c] >= 0 && group_idx[cam_group[c]] == gg.x) u += camp[c * E + e];
+    }
+    part[0][threadIdx.x] = u;
+    part[1][threadIdx.x] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x >= E) return;
+  u = w = 0.0;
+  for (int q = 0; q < NS; ++q) {
+    u += part[0][q * E + e];
+    w += part[1][q * E + e];
+  }
+  const int ci = intr_col[(int64_t)K * groups[gg.x] + i];
+  if (ci < 0) return;
+  if (k < K) {
+    const int cj = intr_col[(int64_t)K * groups[gg.y] + k];
+    if (cj < 0 || cj > ci) return;
+    double d = 0.0;
+    if (ci == cj) {
+      d = fmin(fmax(u, dmin), dmax);
+      diag_c[ci] = d;
+      d /= *radius;
+    }
+    S[(int64_t)ci * ld + cj] = (T)(u - w + d);
+  } else if (gg.x == gg.y && k == K) {
+    rhs[ci] = (T)u;
+  } else if (gg.x == gg.y && gmax_shards) {
+    atomicMax(gmax_shards + (ci & (kGmaxShards - 1)), (unsigned long long)__double_as_longlong(fabs(u / scale_c[ci])));
   }
 }
 
@@ -2259,16 +2493,16 @@ static int key_bits(uint64_t max_key) {
   while (b < 32 && (1ull << b) <= max_key) ++b;
   return b;
 }
-// Camera -> intrinsic group map and the "free intrinsic blocks are private" check.
+// Camera -> intrinsic group map, and what keeps the camera-pair blocks from owning the intrinsics.
 __global__ void k_cam_groups(const uint32_t* cam, const uint32_t* icam, int64_t no, const uint8_t* intr_var,
                              int32_t* cam_group, uint32_t* group_cam, int* conflict, uint32_t* cam_hist) {
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < no; o += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t c = cam[o], g = icam[o];
     const int32_t prev = atomicCAS(&cam_group[c], -1, (int32_t)g);
-    if (prev != -1 && prev != (int32_t)g) atomicExch(conflict, 1);
+    if (prev != -1 && prev != (int32_t)g) atomicExch(conflict, 1);  // a camera of several groups
     if (intr_var[g]) {
       const uint32_t pc = atomicCAS(&group_cam[g], 0xffffffffu, c);
-      if (pc != 0xffffffffu && pc != c) atomicExch(conflict, 1);
+      if (pc != 0xffffffffu && pc != c) atomicExch(conflict + 1, 1);  // a free group of several cameras
     }
     atomicAdd(&cam_hist[c], 1u);
   }
@@ -2717,6 +2951,19 @@ struct Solve {
   uint32_t *blocks = nullptr, *blk_off = nullptr, *cam_off = nullptr, *cam_obs = nullptr;
   unsigned long long* pairs = nullptr;
   int32_t* cam_group = nullptr;
+  // Group of each camera whose columns its blocks hold: cam_group, or -1 for
+  // all where free groups are shared (k_group_*) or no intrinsic is free.
+  int32_t* block_group = nullptr;
+  int bb = 0;                       // rows of a camera-pair block: 6 + k, or 6 without the intrinsics
+  int n_free = 0;                   // free intrinsic groups
+  std::vector<int32_t> group_list;  // host: [ni] index of a free group or -1, then the n_free groups
+  bool shared = false;              // free groups of several cameras
+  int32_t* group_idx = nullptr;
+  int32_t* groups = nullptr;
+  void *grp_g = nullptr, *grp_h = nullptr;
+  unsigned long long* grp_mask = nullptr;
+  double *grp_cam = nullptr, *grp_part = nullptr;
+  int nb_grp = 0;
   void* rec = nullptr;
   bool dense = true;
   int schur_build = GBBA_SCHUR_BUILD_AUTO;  // gbba_options::schur_build
@@ -2945,6 +3192,12 @@ static void setup(gbba_handle* h, const gbba_problem* P, const gbba_options* o, 
   }
   s.n_red = col;
   s.n_pad = ceil_div(std::max<int64_t>(col, 1), kDenseTile) * kDenseTile;
+  s.group_list.assign(ni, -1);
+  for (int64_t g = 0; g < ni; ++g)
+    if (ivar[g]) {
+      s.group_list[g] = s.n_free++;
+      s.group_list.push_back((int32_t)g);
+    }
 
   // counting sort of observations by point (input order kept within a point)
   scan_offsets(h, counts, s.pt_off, np, chunks, st);
@@ -3014,6 +3267,7 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     Arena& A = h->pair_arena;
     Planner p1;
     p1.take<int32_t>(nc);
+    p1.take<int32_t>(nc);
     p1.take<uint32_t>(ni);
     p1.take<int>(2);
     p1.take<uint32_t>(nc + 1);
@@ -3043,6 +3297,7 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     A.reset();
     A.reserve(p1.used + phase2_guess + 4096);
     s.cam_group = A.take<int32_t>(nc);
+    s.block_group = A.take<int32_t>(nc);
     uint32_t* group_cam = A.take<uint32_t>(ni);
     int* conflict = A.take<int>(2);
     uint32_t* cam_hist = A.take<uint32_t>(nc + 1);
@@ -3085,15 +3340,26 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     k_pair_count<<<std::max(1, (int)std::min<int64_t>(ceil_div(np, 128), h->sm_count * 16)), 128, 0, st>>>(s.pt_off, s.cam, np, pcnt);
     check_launch(h);
     scan_offsets(h, pcnt, pair_off, np, chunks, st);
-    int hconf = 0;
+    int hconf[2] = {0, 0};
     uint32_t total = 0;
-    GBBA_CUDA(cudaMemcpyAsync(&hconf, conflict, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GBBA_CUDA(cudaMemcpyAsync(hconf, conflict, sizeof(hconf), cudaMemcpyDeviceToHost, st));
     GBBA_CUDA(cudaMemcpyAsync(&total, pair_off + np, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
-    if (hconf) {
+    // Shared groups: G and H of every point and group, at most twice the
+    // records (6 K np ng values against (9 B + 8) no), and a mask of 64 groups.
+    // Beyond that, and for cameras with several groups, the point-major build.
+    s.shared = hconf[1] != 0;
+    if (hconf[0] ||
+        (s.shared && (!s.dense || s.n_free > 64 || (int64_t)6 * s.k * np * s.n_free > 2 * no * (9 * B + 8)))) {
       setup_atomic_path(h, s, tsize);
       return;
     }
+    // FP64 blocks leave out intrinsics that no camera's block owns (the mixed
+    // path's keep them where they are held: zeros, but its tile's order of sums)
+    const bool ext_only = s.shared || (tsize == 8 && s.dense && s.n_free == 0);
+    if (ext_only) GBBA_CUDA(cudaMemsetAsync(s.block_group, 0xff, sizeof(int32_t) * nc, st));
+    else s.block_group = s.cam_group;
+    s.bb = ext_only ? 6 : B;
     Planner p2;
     if (!want_pairs) total = 0;
     size_t pair_sort_bytes = 0;
@@ -3156,7 +3422,12 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
       count_launch(h, 4);
     }
     // work items: chunks of at most `chunk` (<= kPairChunk) pairs per camera-pair block
-    const uint32_t chunk = (uint32_t)std::min(std::max(h->pair_chunk, 1), kPairChunk);
+    // (FP64: shorter ones, down to 16, until there are 16 for every SM, since a
+    // few warps leave the chip idle: two cameras, 400 points 219 -> 19 us a
+    // launch with 6-row blocks; the mixed path keeps its order of sums)
+    uint32_t chunk = (uint32_t)std::min(std::max(h->pair_chunk, 1), kPairChunk);
+    if (tsize == 8)
+      chunk = std::min(chunk, (uint32_t)std::max<int64_t>(16, ceil_div(ceil_div(total, (int64_t)h->sm_count * 16), 8) * 8));
     std::vector<uint32_t> hoff(nk + 1);
     GBBA_CUDA(cudaMemcpyAsync(hoff.data(), s.blk_off, sizeof(uint32_t) * (nk + 1), cudaMemcpyDeviceToHost, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
@@ -3177,11 +3448,29 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     }
     Arena& I = h->item_arena;
     I.reset();
-    I.reserve(sizeof(PairItem) * items.size() + sizeof(PairMerge) * merges.size() + (size_t)slots * B * B * tsize +
-              4096);
-    s.pair_items = I.take<PairItem>(items.size());
-    s.pair_merges = I.take<PairMerge>(merges.size());
-    s.pair_partial = I.take<char>((size_t)slots * B * B * tsize);
+    const int64_t n_gp = s.shared ? np * s.n_free * s.k * 3 : 0, K = s.k;
+    const int64_t n_pp = (int64_t)s.n_free * (s.n_free + 1) / 2;
+    s.nb_grp = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(np, 8 * (32 / K) * 4), h->sm_count));
+    auto take_items = [&](auto& a) {
+      s.pair_items = a.template take<PairItem>(items.size());
+      s.pair_merges = a.template take<PairMerge>(merges.size());
+      s.pair_partial = a.template take<char>((size_t)slots * s.bb * s.bb * tsize);
+      if (!s.shared) return;
+      s.grp_g = a.template take<char>((size_t)n_gp * tsize);
+      s.grp_h = a.template take<char>((size_t)n_gp * tsize);
+      s.grp_mask = a.template take<unsigned long long>(np);
+      s.grp_cam = a.template take<double>(nc * K * (K + 2));
+      s.grp_part = a.template take<double>((size_t)n_pp * s.nb_grp * K * K);
+      s.group_idx = a.template take<int32_t>(s.group_list.size());
+      s.groups = s.group_idx + ni;
+    };
+    Planner pi;
+    take_items(pi);
+    I.reserve(pi.used + 4096);
+    take_items(I);
+    if (s.shared)
+      GBBA_CUDA(cudaMemcpyAsync(s.group_idx, s.group_list.data(), sizeof(int32_t) * s.group_list.size(),
+                                cudaMemcpyHostToDevice, st));
     GBBA_CUDA(cudaMemcpyAsync(s.pair_items, items.data(), sizeof(PairItem) * items.size(), cudaMemcpyHostToDevice, st));
     GBBA_CUDA(cudaMemcpyAsync(s.pair_merges, merges.data(), sizeof(PairMerge) * merges.size(), cudaMemcpyHostToDevice, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
@@ -3548,32 +3837,57 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
           if (!fp64_inverse) point_rec(std::false_type());
           check_launch(h);
           if (s.dense && s.n_blocks > 0) {
-            auto pairs = [&](auto k) {
-              k_schur_pairs<B, T, decltype(k)::value><<<(unsigned)ceil_div(s.n_blocks * 32, 128), 128, 0, st>>>(
-                  (const PairItem*)s.pair_items, s.n_blocks, s.pairs, (const T*)s.rec, s.ext_col, s.intr_col,
-                  s.cam_group, s.k, s.nc, S, s.n_pad, (T*)s.pair_partial);
+            auto pairs = [&](auto k, auto rows) {
+              constexpr int BB = decltype(rows)::value;
+              k_schur_pairs<B, T, decltype(k)::value, BB>
+                  <<<(unsigned)ceil_div(s.n_blocks * 32, 128), 128, 0, st>>>(
+                      (const PairItem*)s.pair_items, s.n_blocks, s.pairs, (const T*)s.rec, s.ext_col, s.intr_col,
+                      s.block_group, s.k, s.nc, S, s.n_pad, (T*)s.pair_partial);
+              check_launch(h);
+              if (s.n_merges > 0) {
+                k_pair_merge<BB, T><<<(unsigned)ceil_div(s.n_merges * 32, 128), 128, 0, st>>>(
+                    (const PairMerge*)s.pair_merges, s.n_merges, (const T*)s.pair_partial, s.ext_col, s.intr_col,
+                    s.block_group, s.k, s.nc, S, s.n_pad);
+                check_launch(h);
+              }
+            };
+            auto rows = [&](auto k) {
+              if (s.bb == 6) pairs(k, std::integral_constant<int, 6>());
+              else pairs(k, std::integral_constant<int, B>());
             };
             if constexpr (kPose) {
-              if (kahan) pairs(std::true_type());
+              if (kahan) rows(std::true_type());
             }
-            if (!kahan) pairs(std::false_type());
-            check_launch(h);
-            if (s.n_merges > 0) {
-              k_pair_merge<B, T><<<(unsigned)ceil_div(s.n_merges * 32, 128), 128, 0, st>>>(
-                  (const PairMerge*)s.pair_merges, s.n_merges, (const T*)s.pair_partial, s.ext_col, s.intr_col,
-                  s.cam_group, s.k, s.nc, S, s.n_pad);
-              check_launch(h);
-            }
+            if (!kahan) rows(std::false_type());
           }
           if (s.nc > 0) {
             auto rhs_cam = [&](auto compact) {
               k_rhs_camera<B, T, decltype(compact)::value><<<(unsigned)s.nc, kRhsThreads, 0, st>>>(
-                  s.cam_off, s.cam_obs, (const T*)s.rec, s.ext_col, s.intr_col, s.cam_group, s.k, s.nc, rhs,
+                  s.cam_off, s.cam_obs, (const T*)s.rec, s.ext_col, s.intr_col, s.block_group, s.k, s.nc, rhs,
                   s.scale_c, s.diag_c, o->min_lm_diagonal, o->max_lm_diagonal, s.radius, s.dense ? S : nullptr,
                   s.n_pad, gshards);
             };
             if (s.dense) rhs_cam(std::false_type());
             else rhs_cam(std::true_type());
+            check_launch(h);
+          }
+          if (s.shared) {
+            constexpr int K = B - 6;
+            const int ng = s.n_free, n_pp = ng * (ng + 1) / 2;
+            k_group_points<B, T><<<(unsigned)ceil_div(s.np * ng * K, 256), 256, 0, st>>>(
+                s.pt_off, s.icam, s.group_idx, s.np, ng, (const T*)s.rec, (const T*)s.Vinv, (T*)s.grp_g, (T*)s.grp_h,
+                s.grp_mask);
+            check_launch(h);
+            k_group_camera<B, T><<<dim3((unsigned)s.nc, ng + 1), kGroupThreads, 0, st>>>(
+                s.cam_off, s.cam_obs, s.pt, s.cam_group, s.group_idx, s.groups, ng, (const T*)s.rec,
+                (const T*)s.grp_h, s.grp_mask, s.ext_col, s.intr_col, S, s.n_pad, s.grp_cam);
+            check_launch(h);
+            k_group_pairs<K, T><<<dim3(s.nb_grp, n_pp), kGroupThreads, 0, st>>>(
+                s.np, ng, (const T*)s.grp_g, (const T*)s.grp_h, s.grp_mask, s.grp_part);
+            check_launch(h);
+            k_group_merge<K, T><<<n_pp, kGroupThreads, 0, st>>>(
+                s.nc, s.cam_group, s.group_idx, s.groups, s.grp_cam, s.grp_part, s.nb_grp, s.intr_col, S, s.n_pad,
+                rhs, s.scale_c, s.diag_c, o->min_lm_diagonal, o->max_lm_diagonal, s.radius, gshards);
             check_launch(h);
           }
           if (!s.dense && s.nc > 0) {
