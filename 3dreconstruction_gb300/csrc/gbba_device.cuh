@@ -35,19 +35,37 @@ template <typename T> __device__ __forceinline__ void dsincos(T x, T* s, T* c);
 template <> __device__ __forceinline__ void dsincos<double>(double x, double* s, double* c) { sincos(x, s, c); }
 template <> __device__ __forceinline__ void dsincos<float>(float x, float* s, float* c) { sincosf(x, s, c); }
 
-// p = R(w) X  with R, and dp/dw when kJac.
-template <typename T, bool kJac>
-__device__ __forceinline__ void rotate(const T w[3], const T X[3], T p[3], T R[3][3], T dpdw[3][3]) {
+// What a rotation needs of its vector w alone: theta = |w|, u = w / theta, its
+// sine and cosine (big), or w itself in the first-order branch.
+template <typename T>
+struct RotTerms {
+  T s, c, ith, omc, u[3];
+  bool big;
+};
+template <typename T>
+__device__ __forceinline__ RotTerms<T> rot_terms(const T w[3]) {
+  RotTerms<T> q{T(0), T(0), T(0), T(0), {w[0], w[1], w[2]}, false};
   const T th2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
   if (th2 > T(DBL_EPSILON)) {
     const T th = dsqrt(th2);
-    T s, c;
-    dsincos(th, &s, &c);
-    const T ith = T(1) / th;
-    const T u[3] = {w[0] * ith, w[1] * ith, w[2] * ith};
+    dsincos(th, &q.s, &q.c);
+    q.ith = T(1) / th;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) q.u[i] = w[i] * q.ith;
+    q.omc = T(1) - q.c;
+    q.big = true;
+  }
+  return q;
+}
+
+// p = R(w) X  with R, and dp/dw when kJac.
+template <typename T, bool kJac>
+__device__ __forceinline__ void rotate_by(const RotTerms<T>& q, const T X[3], T p[3], T R[3][3], T dpdw[3][3]) {
+  if (q.big) {
+    const T s = q.s, c = q.c, ith = q.ith, omc = q.omc;
+    const T u[3] = {q.u[0], q.u[1], q.u[2]};
     const T uxX[3] = {u[1] * X[2] - u[2] * X[1], u[2] * X[0] - u[0] * X[2], u[0] * X[1] - u[1] * X[0]};
     const T udX = u[0] * X[0] + u[1] * X[1] + u[2] * X[2];
-    const T omc = T(1) - c;
     const T tmp = udX * omc;
 #pragma unroll
     for (int i = 0; i < 3; ++i) p[i] = X[i] * c + uxX[i] * s + u[i] * tmp;
@@ -72,6 +90,7 @@ __device__ __forceinline__ void rotate(const T w[3], const T X[3], T p[3], T R[3
     }
   } else {
     // first-order branch: R p = p + w x p
+    const T w[3] = {q.u[0], q.u[1], q.u[2]};
     p[0] = X[0] + (w[1] * X[2] - w[2] * X[1]);
     p[1] = X[1] + (w[2] * X[0] - w[0] * X[2]);
     p[2] = X[2] + (w[0] * X[1] - w[1] * X[0]);
@@ -84,6 +103,11 @@ __device__ __forceinline__ void rotate(const T w[3], const T X[3], T p[3], T R[3
       dpdw[2][0] = X[1];  dpdw[2][1] = -X[0]; dpdw[2][2] = T(0);
     }
   }
+}
+
+template <typename T, bool kJac>
+__device__ __forceinline__ void rotate(const T w[3], const T X[3], T p[3], T R[3][3], T dpdw[3][3]) {
+  rotate_by<T, kJac>(rot_terms<T>(w), X, p, R, dpdw);
 }
 
 // Camera model applied to the camera-frame point p: residual, and with kJac
@@ -153,14 +177,17 @@ __device__ __forceinline__ void camera_residual(const T* __restrict__ Kp, const 
 
 // Residual (and Jacobian blocks when kJac) of one observation.
 //   Je [2][6]: d r / d(w, t);  Jk [2][K]: d r / d intrinsics;  Jx [2][3]: d r / d X
+// From the terms of the camera's rotation and its translation t, or from its
+// extrinsics E.
 template <int M, typename T, bool kJac>
-__device__ __forceinline__ void residual(const T* __restrict__ Kp, const T E[6], const T X[3], T ox, T oy,
-                                         T r[2], T Je[2][6], T Jk[2][Model<M>::K], T Jx[2][3], T* depth) {
+__device__ __forceinline__ void residual_by(const T* __restrict__ Kp, const RotTerms<T>& q, const T t[3], const T X[3],
+                                            T ox, T oy, T r[2], T Je[2][6], T Jk[2][Model<M>::K], T Jx[2][3],
+                                            T* depth) {
   T p[3], R[3][3], dpdw[3][3];
-  rotate<T, kJac>(E, X, p, R, dpdw);
-  p[0] += E[3];
-  p[1] += E[4];
-  p[2] += E[5];
+  rotate_by<T, kJac>(q, X, p, R, dpdw);
+  p[0] += t[0];
+  p[1] += t[1];
+  p[2] += t[2];
   if (depth) *depth = p[2];
   T D[2][3];
   camera_residual<M, T, kJac>(Kp, p, ox, oy, r, Jk, D);
@@ -176,6 +203,18 @@ __device__ __forceinline__ void residual(const T* __restrict__ Kp, const T E[6],
     }
   }
 }
+template <int M, typename T, bool kJac>
+__device__ __forceinline__ void residual(const T* __restrict__ Kp, const T E[6], const T X[3], T ox, T oy,
+                                         T r[2], T Je[2][6], T Jk[2][Model<M>::K], T Jx[2][3], T* depth) {
+  residual_by<M, T, kJac>(Kp, rot_terms<T>(E), E + 3, X, ox, oy, r, Je, Jk, Jx, depth);
+}
+
+// The FP32 Jacobian's camera data in one row of float4s: rotation terms, t,
+// intrinsics and the Jacobi scales of the camera-side columns (0 = held).
+template <int K>
+struct CamRow {
+  static constexpr int kT = 8, kK = 11, kS = 11 + K, kSize = (11 + K + 6 + K + 3) / 4 * 4;
+};
 
 // Camera pose as 12 values: R(w) row-major (the matrix form of the rotation
 // that rotate() applies, with the same first-order branch) and t.
