@@ -171,6 +171,10 @@ struct Prob {
   // writes them.
   const float4* rc;
   float4* rc_out;
+  // The corrected residual and sqrt(rho') in FP64 (3 per observation) from the
+  // first cost pass, or null: read by the first linearisation.
+  const double* r64;
+  double* r64_out;
 };
 
 template <int M, typename T>
@@ -182,6 +186,11 @@ struct ObsJac {
   T Jp[2][3];       // corrected point block
   int32_t col[B];   // reduced column of each camera-side coordinate (-1 = held)
 };
+
+// isfinite and v > 0 without an operation of the FP64 pipe (64 cycles each for a
+// warp on GB300).
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ unsigned long long max_bits(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
 // n (a multiple of 4) consecutive FP32 values from a 16-byte aligned address,
 // in 16-byte loads issued together.
@@ -245,9 +254,9 @@ __device__ __forceinline__ void obs_jacobian(const Prob& P, int64_t o, const dou
   for (int i = 0; i < K; ++i) Kd[i] = __ldg(&P.intr[K * (int64_t)g + i]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) Xd[i] = __ldg(&P.pts[3 * (int64_t)p + i]);
+  double sr1 = -1.0;  // >= 0: r is already corrected
   T Je[2][6], Jk[2][K], Jx[2][3];
   double r[2];
-  double r_sr1 = -1.0;  // >= 0: r is already corrected and this is sqrt(rho') (residual cache)
   bool done = false;
   if constexpr (sizeof(T) == 8 && kLin) {
     done = P.lin != nullptr;
@@ -265,7 +274,11 @@ __device__ __forceinline__ void obs_jacobian(const Prob& P, int64_t o, const dou
       const float4 q = __ldg(&P.rc[o]);
       r[0] = q.x;
       r[1] = q.y;
-      r_sr1 = q.z;
+      sr1 = q.z;
+    } else if (P.r64) {
+      r[0] = P.r64[3 * o];
+      r[1] = P.r64[3 * o + 1];
+      sr1 = P.r64[3 * o + 2];
     } else if (P.pose) {
       residual_pose<M, double>(Kd, P.pose + 12 * (int64_t)c, Xd, ob.x, ob.y, r);
     } else {
@@ -291,9 +304,7 @@ __device__ __forceinline__ void obs_jacobian(const Prob& P, int64_t o, const dou
     }
     residual<M, T, true>(Kf, Ef, Xf, (T)ob.x, (T)ob.y, rf, Je, Jk, Jx, (T*)nullptr);
   }
-  double sr1;
-  if (r_sr1 >= 0.0) {
-    sr1 = r_sr1;
+  if (sr1 >= 0.0) {
     *cost = 0.0;  // not evaluated: the cost pass has it
     J.r[0] = r[0];
     J.r[1] = r[1];
@@ -350,7 +361,7 @@ __global__ void __launch_bounds__(256) k_linearize_max(Prob P, unsigned long lon
       // |v| as ordered bits; a non-finite term keeps the all-ones word (the
       // sums of its column become NaN)
       const double a = fabs(v);
-      atomicMax(p, isfinite(a) ? (unsigned long long)__double_as_longlong(a) : ~0ull);
+      atomicMax(p, finite_bits(a) ? (unsigned long long)__double_as_longlong(a) : ~0ull);
     };
 #pragma unroll
     for (int j = 0; j < B; ++j) {
@@ -369,22 +380,20 @@ __global__ void __launch_bounds__(256) k_linearize_max(Prob P, unsigned long lon
   }
 }
 
-// Per column: the two exponents (norm, gradient) packed into one double of
+// Per column: the two exponents (norm, gradient) as the two words of a double of
 // the LM-diagonal array (free until k_scale_diag rewrites it), and the
 // accumulators cleared.
 __global__ void k_linearize_exp(int64_t n, double nobs, unsigned long long* __restrict__ mn,
                                 unsigned long long* __restrict__ mg, double* __restrict__ exps) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int en = lin_exp(mn[i], nobs), eg = lin_exp(mg[i], nobs);
-    exps[i] = (double)(en + 8192) * 16384.0 + (double)(eg + 8192);
+    exps[i] = __hiloint2double(lin_exp(mn[i], nobs), lin_exp(mg[i], nobs));
     mn[i] = 0ull;
     mg[i] = 0ull;
   }
 }
 __device__ __forceinline__ void lin_unpack(double packed, int& en, int& eg) {
-  const int hi = (int)(packed / 16384.0);
-  en = hi - 8192;
-  eg = (int)(packed - (double)hi * 16384.0) - 8192;
+  en = __double2hiint(packed);
+  eg = __double2loint(packed);
 }
 template <int M, typename T>
 __global__ void __launch_bounds__(256) k_linearize(Prob P, double* __restrict__ cn_c, double* __restrict__ cn_p,
@@ -602,10 +611,10 @@ using RecOf = typename std::conditional<kCompact, RecC<B>, Rec<B>>::type;
 // (V + D_p^2 / radius)^-1 of one point by a 3x3 Cholesky; v = upper
 // triangle of V (00 01 02 11 12 22).  Returns false on a non-positive pivot
 // or a non-finite inverse.
+// damp = D_p^2 / radius in the compute type.
 template <typename T>
-__device__ __forceinline__ bool point_vinv(const T v[6], const double* __restrict__ dp, double rad, T vi[6],
-                                           T* pivot_ratio = nullptr) {
-  const T a00 = v[0] + (T)(dp[0] / rad), a11 = v[3] + (T)(dp[1] / rad), a22 = v[5] + (T)(dp[2] / rad);
+__device__ __forceinline__ bool point_vinv(const T v[6], const T damp[3], T vi[6], T* pivot_ratio = nullptr) {
+  const T a00 = v[0] + damp[0], a11 = v[3] + damp[1], a22 = v[5] + damp[2];
   const T l00 = sqrt(a00), l10 = v[1] / l00, l20 = v[2] / l00;
   const T d1 = a11 - l10 * l10;
   const T l11 = sqrt(d1), l21 = (v[4] - l20 * l10) / l11;
@@ -677,11 +686,11 @@ __global__ void k_pt_groups(const uint32_t* __restrict__ pt_off, int64_t np, con
 constexpr int kGmaxShards = 64;
 __device__ __forceinline__ void gmax_update(unsigned long long* shards, double m) {
   if (!shards) return;  // no gradient tolerance: the norm is not needed
+  unsigned long long b = (unsigned long long)__double_as_longlong(m);  // m >= 0: ordered as its bits
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.0)
-    atomicMax(shards + (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) & (kGmaxShards - 1)),
-              (unsigned long long)__double_as_longlong(m));
+  for (int o = 16; o > 0; o >>= 1) b = max_bits(b, __shfl_xor_sync(0xffffffffu, b, o));
+  if ((threadIdx.x & 31) == 0 && b != 0)
+    atomicMax(shards + (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) & (kGmaxShards - 1)), b);
 }
 
 template <int M, typename T, bool kFp64Inverse = false, bool kCompact = false>
@@ -737,18 +746,51 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 1) k_schur_point_rec
     for (int i = 0; i < 6; ++i) v[i] = __shfl_sync(0xffffffffu, v[i], tail);
 #pragma unroll
     for (int i = 0; i < 3; ++i) g[i] = __shfl_sync(0xffffffffu, g[i], tail);
+    auto clamp = [&](T d) { return fmin(fmax((double)d, dmin), dmax); };
     double gm = 0.0;
-    if (gmax_shards && valid && lane == head) {
+    T damp[3];
+    if constexpr (sizeof(T) == 4) {
+      // the group's FP64 work: lane e takes value j of point i, e = 3 i + j, of
+      // the points' first lanes, so that a warp divides once or twice (damping,
+      // gradient norm) instead of six times
+      const int ne = 3 * (int)(p1 - p0), mine = 3 * (int)(p - p0);
+      for (int e0 = 0; e0 < ne; e0 += 32) {
+        const int e = e0 + lane, i = e / 3, j = e - 3 * i;
+        const bool in = e < ne;
+        const int from = in ? (int)(P.pt_off[p0 + i] - o0) : 0;
+        const T v0 = __shfl_sync(0xffffffffu, v[0], from), v3 = __shfl_sync(0xffffffffu, v[3], from),
+                v5 = __shfl_sync(0xffffffffu, v[5], from);
+        const double d = clamp(j == 0 ? v0 : j == 1 ? v3 : v5);
+        if (in) diag_p[3 * (int64_t)p0 + e] = d;
+        const T q = (T)(d / rad);
+        if (gmax_shards) {
+          const T g0 = __shfl_sync(0xffffffffu, g[0], from), g1 = __shfl_sync(0xffffffffu, g[1], from),
+                  g2 = __shfl_sync(0xffffffffu, g[2], from);
+          if (in) gm = fmax(gm, fabs((double)(j == 0 ? g0 : j == 1 ? g1 : g2) / scale_p[3 * (int64_t)p0 + e]));
+        }
 #pragma unroll
-      for (int j = 0; j < 3; ++j) gm = fmax(gm, fabs((double)g[j] / scale_p[3 * (int64_t)p + j]));
+        for (int c = 0; c < 3; ++c) {
+          const T y = __shfl_sync(0xffffffffu, q, (mine + c) & 31);
+          if ((unsigned)(mine + c - e0) < 32u) damp[c] = y;
+        }
+      }
+    } else {
+      const double dp[3] = {clamp(v[0]), clamp(v[3]), clamp(v[5])};
+      if (gmax_shards && valid && lane == head) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) gm = fmax(gm, fabs((double)g[j] / scale_p[3 * (int64_t)p + j]));
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        damp[j] = (T)(dp[j] / rad);
+        if (valid && lane == head) diag_p[3 * (int64_t)p + j] = dp[j];
+      }
     }
     gmax_update(gmax_shards, gm);
     // lanes past the group's observations stay (the record copy below is
     // the warp's); their side effects are masked
-    const double dp[3] = {fmin(fmax((double)v[0], dmin), dmax), fmin(fmax((double)v[3], dmin), dmax),
-                          fmin(fmax((double)v[5], dmin), dmax)};
     T vi[6], pr = T(1);
-    bool ok = point_vinv<T>(v, dp, rad, vi, &pr);
+    bool ok = point_vinv<T>(v, damp, vi, &pr);
     if constexpr (sizeof(T) == 4 && kFp64Inverse) {
       // FP32 pivots spanning more than 1e4: V again from an FP64 Jacobian,
       // summed and inverted in FP64 (the point's lanes; the warp's scan)
@@ -774,7 +816,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 1) k_schur_point_rec
         for (int i = 0; i < 6; ++i) v64[i] = __shfl_sync(0xffffffffu, v64[i], tail);
         if (bad) {
           double vi64[6];
-          ok = point_vinv<double>(v64, dp, rad, vi64);
+          const double d64[3] = {clamp(v[0]) / rad, clamp(v[3]) / rad, clamp(v[5]) / rad};
+          ok = point_vinv<double>(v64, d64, vi64);
 #pragma unroll
           for (int i = 0; i < 6; ++i) vi[i] = (T)vi64[i];
         }
@@ -785,10 +828,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 1) k_schur_point_rec
 #pragma unroll
       for (int i = 0; i < 6; ++i) Vinv[6 * (int64_t)p + i] = vi[i];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        gp[3 * (int64_t)p + i] = g[i];
-        diag_p[3 * (int64_t)p + i] = dp[i];
-      }
+      for (int i = 0; i < 3; ++i) gp[3 * (int64_t)p + i] = g[i];
     }
     const T Vf[3][3] = {{vi[0], vi[1], vi[2]}, {vi[1], vi[3], vi[4]}, {vi[2], vi[4], vi[5]}};
     const T r0 = (T)J.r[0], r1 = (T)J.r[1];
@@ -1030,8 +1070,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 1) k_schur_point_rec
   gmax_update(gmax_shards, gm);
   const double dp[3] = {fmin(fmax((double)v[0], dmin), dmax), fmin(fmax((double)v[3], dmin), dmax),
                         fmin(fmax((double)v[5], dmin), dmax)};
+  const T damp[3] = {(T)(dp[0] / rad), (T)(dp[1] / rad), (T)(dp[2] / rad)};
   T vi[6];
-  const bool ok = point_vinv<T>(v, dp, rad, vi);
+  const bool ok = point_vinv<T>(v, damp, vi);
   if (lane == 0) {
     if (!ok) atomicExch(flag, 2);
 #pragma unroll
@@ -2606,7 +2647,9 @@ __global__ void __launch_bounds__(128) k_backsub_rec(const uint32_t* __restrict_
     const T q0 = gp[3 * (int64_t)p] - t[0], q1 = gp[3 * (int64_t)p + 1] - t[1], q2 = gp[3 * (int64_t)p + 2] - t[2];
     y[0] = vi[0] * q0 + vi[1] * q1 + vi[2] * q2;
     y[1] = vi[1] * q0 + vi[3] * q1 + vi[4] * q2;
-    y[2] = vi[2] * q0 + vi[4] * q1 + vi[5] * q2;
+    // spelled out: a mixed solve's results hang on the last bit of a point, and
+    // the compiler's choice of the product that is rounded varied here
+    y[2] = fma(vi[5], q2, fma(vi[2], q0, vi[4] * q1));
   };
   if (w < n_groups) {
     const uint32_t p0 = pt_grp[w], p1 = pt_grp[w + 1];
@@ -2660,19 +2703,36 @@ __global__ void __launch_bounds__(128) k_backsub_rec(const uint32_t* __restrict_
       }
 #pragma unroll
       for (int j = 0; j < 3; ++j) t[j] = __shfl_sync(0xffffffffu, t[j], tail);
+      T y[3] = {T(0), T(0), T(0)};
       if (valid) {
-        T y[3];
         point_step(p, t, y);
         mcc = obs_mcc(vw, f0, f1, y);
-        if (lane == head) {
-          if (!isfinite(y[0]) || !isfinite(y[1]) || !isfinite(y[2])) atomicExch(flag, 3);
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            const double d = -(double)y[j] * scale_p[3 * (int64_t)p + j];
-            pts_new[3 * (int64_t)p + j] = pts[3 * (int64_t)p + j] + d;
-            stp += d * d;
-          }
+        if (lane == head && (!isfinite(y[0]) || !isfinite(y[1]) || !isfinite(y[2]))) atomicExch(flag, 3);
+      }
+      // candidate points: lane e takes coordinate j of point i, e = 3 i + j (a
+      // third of the FP64 instructions, and coalesced)
+      const int ne = 3 * (int)(p1 - p0), mine = 3 * (int)(p - p0);
+      double d[3];
+      for (int e0 = 0; e0 < ne; e0 += 32) {
+        const int e = e0 + lane, i = e / 3, j = e - 3 * i;
+        const bool in = e < ne;
+        const int from = in ? (int)(pt_off[p0 + i] - o0) : 0;
+        const T y0 = __shfl_sync(0xffffffffu, y[0], from), y1 = __shfl_sync(0xffffffffu, y[1], from),
+                y2 = __shfl_sync(0xffffffffu, y[2], from);
+        double de = 0.0;
+        if (in) {
+          de = -(double)(j == 0 ? y0 : j == 1 ? y1 : y2) * scale_p[3 * (int64_t)p0 + e];
+          pts_new[3 * (int64_t)p0 + e] = pts[3 * (int64_t)p0 + e] + de;
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double x = __shfl_sync(0xffffffffu, de, (mine + c) & 31);
+          if ((unsigned)(mine + c - e0) < 32u) d[c] = x;
+        }
+      }
+      if (valid && lane == head) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) stp += d[j] * d[j];
       }
     } else {
       // one point (no observation, or more than 32)
@@ -2705,12 +2765,12 @@ __global__ void __launch_bounds__(128) k_backsub_rec(const uint32_t* __restrict_
       }
     }
   }
-  mcc = warp_sum(mcc);
-  stp = warp_sum(stp);
-  if (lane == 0) {
-    smcc[warp] = mcc;
-    sstep[warp] = stp;
-  }
+  // both sums at once: the lower half of the warp takes mcc, the upper stp
+  double both = (lane < 16 ? mcc : stp) + __shfl_xor_sync(0xffffffffu, lane < 16 ? stp : mcc, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) both += __shfl_xor_sync(0xffffffffu, both, o);
+  if (lane == 0) smcc[warp] = both;
+  if (lane == 16) sstep[warp] = both;
   __syncthreads();
   if (threadIdx.x == 0) {
     part_mcc[blockIdx.x] = smcc[0] + smcc[1] + smcc[2] + smcc[3];
@@ -2892,33 +2952,82 @@ __global__ void __launch_bounds__(64) k_cam_row(const float* __restrict__ ext_f,
 }
 
 // FP64 robustified cost 1/2 sum rho(|r|^2) at (ext, intr, pts); per-block partials.
+// Bound by the FP64 pipe.  The robust loss's roots and quotient (a third of the
+// instructions when each warp with one outlier takes them) are evaluated for
+// the outliers of four observations a thread at once, in their packed order;
+// every thread still adds its costs in the order of its observations.
 template <int M>
 __global__ void __launch_bounds__(256) k_cost(Prob P, const double* ext, const double* intr, const double* pts,
                                               double* part_cost, int* nonfinite) {
   constexpr int K = Model<M>::K;
+  constexpr int U = 4;
   __shared__ double sh[8];
+  __shared__ double2 rob[8][32 * U];  // outliers of a warp's round: |r|^2, then cost and sqrt(rho')
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const long long a2 = P.loss_type == 1 ? __double_as_longlong(P.loss_a * P.loss_a) : 0x7fffffffffffffffll;
   double acc = 0.0;
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < P.no; o += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = P.cam[o], g = P.icam[o], p = P.pt[o];
-    double E[6], Kp[K], X[3], r[2];
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; w0 < P.no; w0 += U * stride) {
+    double r[U][2], s[U];
+    uint32_t rank[U], total = 0;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) E[i] = __ldg(&ext[6 * (int64_t)c + i]);
+    for (int u = 0; u < U; ++u) {
+      const int64_t o = w0 + lane + u * stride;
+      bool outlier = false;
+      s[u] = r[u][0] = r[u][1] = 0.0;
+      if (o < P.no) {
+        const uint32_t c = P.cam[o], g = P.icam[o], p = P.pt[o];
+        double Kp[K], X[3];
 #pragma unroll
-    for (int i = 0; i < K; ++i) Kp[i] = __ldg(&intr[K * (int64_t)g + i]);
+        for (int i = 0; i < K; ++i) Kp[i] = __ldg(&intr[K * (int64_t)g + i]);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) X[i] = __ldg(&pts[3 * (int64_t)p + i]);
-    const double2 ob = P.obs[o];
-    if (P.pose) {
-      residual_pose<M, double>(Kp, P.pose + 12 * (int64_t)c, X, ob.x, ob.y, r);
-    } else {
-      double dJe[2][6], dJk[2][K], dJx[2][3];
-      residual<M, double, false>(Kp, E, X, ob.x, ob.y, r, dJe, dJk, dJx, (double*)nullptr);
+        for (int i = 0; i < 3; ++i) X[i] = __ldg(&pts[3 * (int64_t)p + i]);
+        const double2 ob = P.obs[o];
+        if (P.pose) {
+          residual_pose<M, double>(Kp, P.pose + 12 * (int64_t)c, X, ob.x, ob.y, r[u]);
+        } else {
+          double E[6], dJe[2][6], dJk[2][K], dJx[2][3];
+#pragma unroll
+          for (int i = 0; i < 6; ++i) E[i] = __ldg(&ext[6 * (int64_t)c + i]);
+          residual<M, double, false>(Kp, E, X, ob.x, ob.y, r[u], dJe, dJk, dJx, (double*)nullptr);
+        }
+        s[u] = r[u][0] * r[u][0] + r[u][1] * r[u][1];
+        outlier = __double_as_longlong(s[u]) > a2;  // both non-negative: ordered as their bits
+      }
+      const uint32_t m = __ballot_sync(0xffffffffu, outlier);
+      rank[u] = outlier ? total + __popc(m & ((1u << lane) - 1u)) : ~0u;
+      if (outlier) rob[warp][rank[u]].x = s[u];
+      total += __popc(m);
     }
-    double sr1;
-    const double cst = robust<double>(P.loss_type, P.loss_a, r[0] * r[0] + r[1] * r[1], &sr1);
-    if (!isfinite(cst)) atomicExch(nonfinite, 1);
-    if (P.rc_out) P.rc_out[o] = make_float4((float)(r[0] * sr1), (float)(r[1] * sr1), (float)sr1, 0.0f);
-    acc += cst;
+    __syncwarp();
+    for (uint32_t k = lane; k < total; k += 32) {
+      double sr1;
+      const double cst = robust<double>(P.loss_type, P.loss_a, rob[warp][k].x, &sr1);
+      rob[warp][k] = make_double2(cst, sr1);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t o = w0 + lane + u * stride;
+      if (o >= P.no) break;
+      double cst = 0.5 * s[u], sr1 = 1.0;
+      if (rank[u] != ~0u) {
+        const double2 q = rob[warp][rank[u]];
+        cst = q.x;
+        sr1 = q.y;
+        r[u][0] *= sr1;
+        r[u][1] *= sr1;
+      }
+      if (!finite_bits(cst)) atomicExch(nonfinite, 1);
+      if (P.rc_out) P.rc_out[o] = make_float4((float)r[u][0], (float)r[u][1], (float)sr1, 0.0f);
+      if (P.r64_out) {
+        P.r64_out[3 * o] = r[u][0];
+        P.r64_out[3 * o + 1] = r[u][1];
+        P.r64_out[3 * o + 2] = sr1;
+      }
+      acc += cst;
+    }
+    __syncwarp();
   }
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
@@ -3072,6 +3181,8 @@ static Prob make_prob(const Solve& s, const double* ext, const double* intr, con
   P.ext_f = P.intr_f = P.pts_f = P.scale_cf = P.scale_pf = P.row = nullptr;
   P.rc = nullptr;
   P.rc_out = nullptr;
+  P.r64 = nullptr;
+  P.r64_out = nullptr;
   return P;
 }
 
@@ -3714,8 +3825,12 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
       check_launch(h);
     }
   };
-  auto launch_cost = [&](const double* e, const double* i, const double* p) {
+  // The first linearisation reads FP64 residuals that the first cost pass
+  // leaves in the (not yet used) records, at least 30 words an observation.
+  double* const r64 = kPose && s.pair_path ? (double*)s.rec : nullptr;
+  auto launch_cost = [&](const double* e, const double* i, const double* p, double* r64_out = nullptr) {
     Prob Pc = make_prob(s, e, i, p, o);
+    Pc.r64_out = r64_out;
     // the mixed path's residual cache: current parameters in slot 0, the
     // candidate in slot 1 (copied to slot 0 when the step is accepted)
     if (kPose && s.rcache) Pc.rc_out = s.rcache + (e == s.ext ? 0 : s.no);
@@ -3740,6 +3855,7 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
       P.ext_f = s.ext_f;
       P.intr_f = s.intr_f;
       P.pts_f = s.pts_f;
+      if (first) P.r64 = r64;
     }
     GBBA_CUDA(cudaMemsetAsync(s.cn_c, 0, sizeof(double) * (s.n_red + 1), st));
     GBBA_CUDA(cudaMemsetAsync(s.g_c, 0, sizeof(double) * (s.n_red + 1), st));
@@ -3829,7 +3945,7 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
 
   // initial cost
   GBBA_CUDA(cudaMemsetAsync(s.nonfinite, 0, sizeof(int), st));
-  launch_cost(s.ext, s.intr, s.pts);
+  launch_cost(s.ext, s.intr, s.pts, r64);
   k_reduce3<<<1, 256, 0, st>>>(s.part_cost, s.nb_obs, s.part_cost, 0, s.part_cost, 0, s.part_cost, 0, s.scalars);
   check_launch(h);
   int nonfinite = 0;
