@@ -30,9 +30,12 @@
 //   - the Cholesky factorisation and both triangular solves run where S
 //     lives; every thread evaluates the step and takes the same accept /
 //     reject decision.
-// CTAs never wait on each other, so the launch cannot deadlock; the hardware
-// schedules the next problem onto an SM as soon as one finishes (problems are
-// ordered largest first to shorten the tail).
+// CTAs of different problems never wait on each other, and the two or four CTAs
+// that share a large problem's Schur build in the mixed path are a cluster,
+// resident together, that meets at the hardware's cluster barriers only; the
+// hardware schedules the next problem onto an SM as soon as one finishes
+// (problems are ordered largest first to shorten the tail).
+#include <cooperative_groups.h>
 #include <math_constants.h>
 
 #include <algorithm>
@@ -81,6 +84,7 @@ struct BOut {
 struct BArgs {
   const BProb* probs;
   const uint32_t* order;
+  uint32_t slot0;  // scratch slice of the launch's first CTA
   double *ext, *intr, *pts, *ext2, *intr2, *pts2;
   const double2* obs;
   const uint32_t *cam, *icam, *pt_off, *pt_s;  // pt_s: point of each (sorted) observation
@@ -153,6 +157,10 @@ struct Shared {
   int32_t fxe[N];  // its exponent (FP64)
   int fxbits;      // S's budget: 2^(2 e_i) bound_i < 2^fxbits
   int fxbad;       // a term out of range or not finite (FP64)
+  // a cluster's first CTA to its helpers: 1 = build, 0 = done, the current
+  // residual cache and 1 / radius; a helper to the first: its points' gradient norm
+  int cmd, cur;
+  double irad, hgm;
   double red[kWarps];
   double bcast[8];
   int flag;
@@ -245,6 +253,11 @@ __device__ __forceinline__ void fx_add(long long* p, double v, int k, int* bad) 
 __device__ __forceinline__ void fx_add(long long* p, float v, float scale) {
   atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__float2ll_rn(v * scale));
 }
+// max(m, v) of non-negative doubles on their bits (a NaN v is left out, as by fmax)
+__device__ __forceinline__ unsigned long long max_nonneg(unsigned long long m, double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b > m && b <= 0x7ff0000000000000ull ? b : m;
+}
 
 // Linearisation of observation o (point p) at the current parameters: the
 // corrected residual rr and Jacobian blocks (compute type) and the reduced
@@ -305,6 +318,21 @@ __device__ __forceinline__ void obs_lin(const BArgs& a, int64_t o, uint32_t p, c
   }
 }
 
+__device__ __forceinline__ uint32_t cluster_ctas() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Every thread of every CTA of the cluster; orders shared and global memory.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // T: Jacobians and point blocks; SS: the shared-memory S, its factor and the step.
 template <int M, typename T, typename SS>
 __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
@@ -313,7 +341,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
   constexpr bool kGS = SharedOf<SS>::kGlobalS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename SharedOf<SS>::type& sh = *reinterpret_cast<typename SharedOf<SS>::type*>(smem_raw);
-  const uint32_t pid = a.order[blockIdx.x];
+  // A cluster of R CTAs owns the window (R = 1 without one): the first runs the
+  // solve, the others build S over their share of the points and hand it over.
+  const uint32_t R = kGS ? 1u : cluster_ctas(), rank = kGS ? 0u : cluster_rank();
+  const bool helper = rank != 0;
+  const uint32_t pid = a.order[blockIdx.x / R];
   const BProb P = a.probs[pid];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = (int)P.n;
@@ -323,9 +355,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
   // one more slot holds per-point sums
   using SL = Slot<K>;
   constexpr int KK = SL::KK;
-  T* wsc = (T*)a.wscratch + ((int64_t)blockIdx.x * kWarps + warp) * (int64_t)(a.max_views + 1) * SL::kSize;
+  T* wsc = (T*)a.wscratch + ((int64_t)(a.slot0 + blockIdx.x) * kWarps + warp) * (int64_t)(a.max_views + 1) * SL::kSize;
   // global slice: column norms [kNMax], gradient [kNMax], rhs [kNMax], S (FP64)
-  double* gsl = a.gscr + (int64_t)blockIdx.x * kGlobalSlice;
+  double* gsl = a.gscr + (int64_t)(a.slot0 + blockIdx.x) * kGlobalSlice;
   double* g_acc = gsl;
   double* g_grad = gsl + kNMax;
   double* g_rhs = gsl + 2 * kNMax;
@@ -511,7 +543,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
     // Column norms and gradient are fixed-point sums (order-independent).
     // Pass 1 finds the largest single term of each, which with the window's
     // observation count bounds every partial sum; pass 2 accumulates.
-    double mc = 0.0, mg = 0.0;
+    unsigned long long bc = 0, bg = 0;
     for (uint32_t p = P.x0 + warp; p < P.x1; p += kWarps) {
       for (uint32_t o = a.pt_off[p] + lane; o < a.pt_off[p + 1]; o += 32) {
         T rr[2], Jc[2][B], Jp[2][3];
@@ -521,13 +553,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
         for (int j = 0; j < B; ++j) {
           if (col[j] < 0) continue;
           const double x0 = Jc[0][j], x1 = Jc[1][j];
-          mc = fmax(mc, x0 * x0 + x1 * x1);
-          mg = fmax(mg, fabs(x0 * (double)rr[0] + x1 * (double)rr[1]));
+          bc = max_nonneg(bc, x0 * x0 + x1 * x1);
+          bg = max_nonneg(bg, fabs(x0 * (double)rr[0] + x1 * (double)rr[1]));
         }
       }
     }
-    mc = block_max(mc, sh.red, &sh.bcast[5]);
-    mg = block_max(mg, sh.red, &sh.bcast[6]);
+    const double mc = block_max(__longlong_as_double((long long)bc), sh.red, &sh.bcast[5]);
+    const double mg = block_max(__longlong_as_double((long long)bg), sh.red, &sh.bcast[6]);
     const double nobs = (double)(a.pt_off[P.x1] - a.pt_off[P.x0]);
     const int kc = pow2_exp(mc * nobs, 62, 1000), kg = pow2_exp(mg * nobs, 62, 1000);
     for (int i = tid; i < n; i += kThreads) {
@@ -588,6 +620,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
     return block_max(gm, sh.red, &sh.bcast[1]);
   };
 
+  // the helpers' last command (they read it between the two barriers)
+  auto release_helpers = [&]() {
+    if (R == 1) return;
+    if (tid == 0) sh.cmd = 0;
+    cluster_sync();
+    cluster_sync();
+  };
+  double cost = 0.0, gmax = 0.0, xnorm = 0.0;
+  BOut res;
+  int term = -1;
+  if (!helper) {
   // the window's column maps, fixed for the whole solve (made visible by make_poses' barrier)
   if (use_pose)
     for (uint32_t i = tid; i < 6 * P.nc; i += kThreads) sh.ecol[i] = a.ext_col[6 * (int64_t)P.c0 + i];
@@ -595,8 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
   make_f32(a.ext, a.intr, a.pts);
   bool finite = true;
   make_poses(a.ext, 0);
-  double cost = cost_at(a.ext, a.intr, a.pts, &finite);
-  BOut res;
+  cost = cost_at(a.ext, a.intr, a.pts, &finite);
   res.initial_cost = cost;
   res.final_cost = cost;
   res.iterations = res.successful = res.unsuccessful = 0;
@@ -608,6 +650,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
       res.status = GBBA_ERROR_NUMERICAL;
       a.out[pid] = res;
     }
+    release_helpers();
     return;
   }
   {
@@ -633,18 +676,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
     if (tid == 0) sh.fxbits = (kGS ? 61 : 30) - (32 - __clz(mult));  // 32 - clz(m) = ceil(log2(1 + m))
     __syncthreads();
   }
-  double gmax = linearize(true), xnorm = param_norm();
+  gmax = linearize(true);
+  xnorm = param_norm();
   {
     // bounds on the scaled column norms for the first build's fixed-point scales
     for (int i = tid; i < n; i += kThreads) sh.cbnd[i] = __ldcg(g_acc + i) * sh.scale_c[i] * sh.scale_c[i];
     __syncthreads();
   }
+  term = gmax <= a.gtol ? GBBA_CONVERGENCE : -1;
+  }  // !helper
   bool check_grad = false;  // an accepted step's gradient is checked by the next Schur build
-  int term = gmax <= a.gtol ? GBBA_CONVERGENCE : -1;
   double radius = a.r0, decrease = 2.0;
   int invalid = 0, iter = 0;
   while (term < 0) {
-    if (iter >= a.max_iterations) {
+    if (!helper && iter >= a.max_iterations) {
       term = GBBA_NO_CONVERGENCE;
       if (check_grad && linearize(false) <= a.gtol) term = GBBA_CONVERGENCE;
       break;
@@ -655,11 +700,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
     // norm of up to 4 cbnd[i] (col_exp gives the bound on S's sums); the
     // vectors with one scale for the window.  A build that finds a column
     // above its bound runs again.
-    const double irad_d = 1.0 / radius;
+    double irad_d = 1.0 / radius;
     T gmt = T(0);  // gradient max norm (unscaled) over this thread's points
     double cover = 0.0;  // largest column norm / its bound of the last build
     for (int attempt = 0;; ++attempt) {
-    {
+    if (!helper) {
       double cb = 0.0;
       for (int i = tid; i < n; i += kThreads) {
         const int e = col_exp(4.0 * sh.cbnd[i], sh.fxbits, kGS ? 500 : 60);
@@ -678,6 +723,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
         for (int q = 1; q < 4; ++q) sh.fx[q] = ldexp(1.0, sh.fxk[q]);
         sh.flag = 0;
         sh.fxbad = 0;
+        sh.cmd = 1;
+        sh.cur = cur;
+        sh.irad = irad_d;
+      }
+    }
+    if (R > 1) {
+      cluster_sync();  // the scales are set
+      if (helper) {
+        const auto* first = cooperative_groups::this_cluster().map_shared_rank(&sh, 0);
+        if (first->cmd == 0) {
+          cluster_sync();
+          return;
+        }
+        for (int i = tid; i < n; i += kThreads) {
+          sh.scale_cf[i] = first->scale_cf[i];
+          sh.fxs[i] = first->fxs[i];
+        }
+        if (use_pose)
+          for (uint32_t i = tid; i < 6 * P.nc; i += kThreads) sh.ecol[i] = first->ecol[i];
+        if (tid < 8) sh.kcol[tid] = first->kcol[tid];
+        if (tid < 4) sh.fx[tid] = first->fx[tid];
+        if (tid == 0) sh.flag = sh.fxbad = 0;
+        cur = first->cur;
+        irad_d = first->irad;
       }
     }
     for (int i = tid; i < n * (n + 1) / 2; i += kThreads) Sst(i, SS(0));
@@ -706,7 +775,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
     // per pair; an observation's own pair carries its U_ee).
     const bool one_group = P.ni == 1;
     const T irad = T(irad_d), dmin = (T)a.dmin, dmax = (T)a.dmax;
-    for (uint32_t p = P.x0 + warp; p < P.x1; p += kWarps) {
+    for (uint32_t p = P.x0 + rank * kWarps + warp; p < P.x1; p += R * kWarps) {
       const uint32_t ob = a.pt_off[p], oe = a.pt_off[p + 1], m = oe - ob;
       const T sp[3] = {psc(p, 0), psc(p, 1), psc(p, 2)};
       T v[6] = {}, g[3] = {};
@@ -798,7 +867,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
       const T i10 = -l10 * i00 * i11, i21 = -l21 * i11 * i22, i20 = -(l20 * i00 + l21 * i10) * i22;
       const T vi[6] = {i00 * i00 + i10 * i10 + i20 * i20, i10 * i11 + i20 * i21, i20 * i22,
                        i11 * i11 + i21 * i21, i21 * i22, i22 * i22};
-      if (!(a00 > T(0)) || !(d1 > T(0)) || !(d2 > T(0)) || !isfinite((double)vi[0])) sh.flag = 2;
+      if (!(a00 > T(0)) || !(d1 > T(0)) || !(d2 > T(0)) || !isfinite(vi[0])) sh.flag = 2;
       if (lane == 0) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) Vinv[6 * (int64_t)p + i] = vi[i];
@@ -941,6 +1010,34 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
       __syncwarp();
     }
     __syncthreads();
+    if constexpr (!kGS) {
+      if (R > 1) {
+        if (helper) {
+          const double g = block_max((double)gmt, sh.red, &sh.bcast[1]);
+          if (tid == 0) sh.hgm = g;
+        }
+        cluster_sync();  // every share of S is complete
+        if (!helper) {
+          for (uint32_t q = 1; q < R; ++q) {
+            const auto* other = cooperative_groups::this_cluster().map_shared_rank(&sh, q);
+            int* mine = reinterpret_cast<int*>(sh.S);
+            const int* theirs = reinterpret_cast<const int*>(other->S);
+            for (int i = tid; i < n * (n + 1) / 2; i += kThreads) mine[i] += theirs[i];
+            for (int i = tid; i < n; i += kThreads) {
+#pragma unroll
+              for (int v = 0; v < 3; ++v) sh.fxv[v][i] += other->fxv[v][i];
+            }
+            gmt = fmax(gmt, (T)other->hgm);
+            if (tid == 0) {
+              if (other->flag) sh.flag = other->flag;
+              sh.fxbad |= other->fxbad;
+            }
+          }
+        }
+        cluster_sync();  // and taken over
+        if (helper) continue;
+      }
+    }
     // the column norms against the bounds the build was scaled for; the
     // next build (this one again, or the next iteration's) takes the norms
     // found as its bounds
@@ -1089,7 +1186,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
       const T q0 = gpv[3 * (int64_t)p] - t[0], q1 = gpv[3 * (int64_t)p + 1] - t[1], q2 = gpv[3 * (int64_t)p + 2] - t[2];
       const T y[3] = {vi[0] * q0 + vi[1] * q1 + vi[2] * q2, vi[1] * q0 + vi[3] * q1 + vi[4] * q2,
                       vi[2] * q0 + vi[4] * q1 + vi[5] * q2};
-      if (!isfinite((double)y[0]) || !isfinite((double)y[1]) || !isfinite((double)y[2])) sh.flag = 3;
+      if (!isfinite(y[0]) || !isfinite(y[1]) || !isfinite(y[2])) sh.flag = 3;
       const T ys[3] = {y[0] * sp[0], y[1] * sp[1], y[2] * sp[2]};
       // model cost change: each term in the compute type, the sum in FP64
       for (uint32_t o = ob + lane; o < oe; o += 32) {
@@ -1174,6 +1271,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lm_batched(BArgs a) {
       if (radius < a.rmin) term = GBBA_CONVERGENCE;
     }
   }
+  release_helpers();
   if (tid == 0) {
     res.termination = term;
     res.usable = term != GBBA_FAILURE ? 1 : 0;
@@ -1373,6 +1471,31 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
   for (int i = 0; i < np_; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(),
                    [&](uint32_t x, uint32_t y) { return (bp[x].o1 - bp[x].o0) > (bp[y].o1 - bp[y].o0); });
+  // Clusters (mixed path): a window's S has to fit one SM, so one CTA used to
+  // build it alone, and a call lasted as long as its largest window while other
+  // SMs had run out of work (304 windows of 5 to 40 cameras: 1.5 times the mean
+  // load of an SM).  The build is 80% of a window's time and its integer sums
+  // do not depend on who adds them: up to a quarter as many windows as SMs get
+  // four CTAs each, up to half as many two, and beyond that the windows of more
+  // than an SM's mean load two.  Two CTAs take 0.6 of the time and so 1.2 times
+  // the SMs': from 0.7 of the mean load on, a call of 304 windows took 182 ms,
+  // from 1.0 on 177, without 215; 100 windows 65.1 -> 42.1 (0.7: 41.0), 20
+  // windows 5.5 -> 3.7 ms.
+  int ctas = 1, clustered = 0;
+  if (!fp64 && np_ > 0) {
+    if (4 * (int64_t)np_ <= h->sm_count) ctas = 4;
+    else ctas = 2;
+    auto load = [&](uint32_t i) {  // observations and their pairs
+      const double o = bp[i].o1 - bp[i].o0;
+      return o * (12.0 + o / std::max<double>(1.0, bp[i].x1 - bp[i].x0));
+    };
+    double sum = 0.0;
+    for (int i = 0; i < np_; ++i) sum += load(i);
+    const double line = 2 * (int64_t)np_ <= h->sm_count ? -1.0 : sum / h->sm_count;
+    clustered = (int)(std::stable_partition(order.begin(), order.end(), [&](uint32_t i) { return load(i) > line; }) -
+                      order.begin());
+  }
+  const int64_t total_ctas = (int64_t)clustered * ctas + (np_ - clustered);
   const int slot_values = k == 1 ? Slot<1>::kSize : k == 6 ? Slot<6>::kSize : Slot<8>::kSize;
   const size_t tsize = 8;  // FP64-sized: the mixed path ends with an FP64 polish
   Planner pl;
@@ -1402,8 +1525,8 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     q.ecol = A.template take<int32_t>(6 * tc); q.icol = A.template take<int32_t>(k * tg); q.ivar = A.template take<uint8_t>(tg);
     q.probs = A.template take<BProb>(np_); q.out = A.template take<BOut>(2 * np_);
     q.Vinv = A.template take<char>(6 * tx * tsize); q.gp = A.template take<char>(3 * tx * tsize);
-    q.wsc = A.template take<char>((size_t)np_ * kWarps * (max_views + 1) * slot_values * tsize);
-    q.gscr = A.template take<double>((size_t)np_ * kGlobalSlice);
+    q.wsc = A.template take<char>((size_t)total_ctas * kWarps * (max_views + 1) * slot_values * tsize);
+    q.gscr = A.template take<double>((size_t)total_ctas * kGlobalSlice);
     q.rcache = A.template take<float4>((size_t)2 * std::max<int64_t>(to, 1));
     q.ext_f = A.template take<float>(6 * tc); q.intr_f = A.template take<float>(k * tg);
     q.pts_f = A.template take<float>(3 * tx); q.scale_pf = A.template take<float>(3 * tx);
@@ -1440,7 +1563,7 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     check_launch(h);
   }
   BArgs a;
-  a.probs = q.probs; a.order = q.order;
+  a.probs = q.probs; a.order = q.order; a.slot0 = 0;
   a.ext = q.ext; a.intr = q.intr; a.pts = q.pts; a.ext2 = q.ext2; a.intr2 = q.intr2; a.pts2 = q.pts2;
   a.obs = q.obs; a.cam = q.cam_s; a.icam = q.icam_s; a.pt_off = q.off;
   a.ext_col = q.ecol; a.intr_col = q.icol; a.intr_var = q.ivar;
@@ -1464,6 +1587,42 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     kern<<<np_, kThreads, smem, st>>>(*base);
     check_launch(h);
   };
+  // the clustered windows on the call's stream, the others beside them
+  auto launch_mixed = [&](auto kern, size_t smem) {
+    if (np_ <= 0) return;
+    GBBA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const bool fork = clustered > 0 && clustered < np_;
+    if (fork) {
+      GBBA_CUDA(cudaEventRecord(h->ev_main, st));
+      GBBA_CUDA(cudaStreamWaitEvent(h->side, h->ev_main, 0));
+    }
+    if (clustered > 0) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)ctas;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)clustered * ctas);
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      GBBA_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+      check_launch(h);
+    }
+    if (clustered < np_) {
+      BArgs rest = a;
+      rest.order = a.order + clustered;
+      rest.slot0 = (uint32_t)(clustered * ctas);
+      kern<<<np_ - clustered, kThreads, smem, fork ? h->side : st>>>(rest);
+      check_launch(h);
+    }
+    if (fork) {
+      GBBA_CUDA(cudaEventRecord(h->ev_side, h->side));
+      GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
+    }
+  };
   // FP64: S in the global slice (small shared footprint); mixed: FP32 S in
   // shared memory
   const size_t sm64 = sizeof(SharedOf<double>::type), sm32 = sizeof(SharedOf<float>::type);
@@ -1472,9 +1631,9 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     else if (model == kRadialK3) launch(k_lm_batched<kRadialK3, double, double>, sm64);
     else launch(k_lm_batched<kBrownT2, double, double>, sm64);
   } else {
-    if (model == kPinholeF) launch(k_lm_batched<kPinholeF, float, float>, sm32);
-    else if (model == kRadialK3) launch(k_lm_batched<kRadialK3, float, float>, sm32);
-    else launch(k_lm_batched<kBrownT2, float, float>, sm32);
+    if (model == kPinholeF) launch_mixed(k_lm_batched<kPinholeF, float, float>, sm32);
+    else if (model == kRadialK3) launch_mixed(k_lm_batched<kRadialK3, float, float>, sm32);
+    else launch_mixed(k_lm_batched<kBrownT2, float, float>, sm32);
   }
   // Mixed path: the FP64 kernel continues from the mixed solution (its own
   // LM restart, at most fp64_polish_iterations iterations, tolerances 1000x
