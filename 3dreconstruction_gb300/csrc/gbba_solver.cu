@@ -60,15 +60,31 @@ static int model_k(int m) { return m == kPinholeF ? 1 : m == kRadialK3 ? 6 : 8; 
 // ------------------------------------------------------------------ setup kernels
 __global__ void k_validate(const uint32_t* cam, const uint32_t* icam, const uint32_t* pt, int64_t no, int64_t nc,
                            int64_t ni, int64_t np, int* err, uint32_t* counts, uint8_t* cam_used, uint8_t* intr_used) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < no; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = cam[i], g = icam[i], p = pt[i];
-    if (c >= nc || g >= ni || p >= np) {
-      atomicExch(err, 1);
-      continue;
+  // observations mostly come point by point: a run of one point inside a warp is
+  // one atomic, and a flag that is set is not written again (20M observations:
+  // 2.9 -> 0.53 ms)
+  const int lane = threadIdx.x & 31;
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; w0 < no; w0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = w0 + lane;
+    bool ok = i < no;
+    uint32_t p = 0;
+    if (ok) {
+      const uint32_t c = cam[i], g = icam[i];
+      p = pt[i];
+      if (c >= nc || g >= ni || p >= np) {
+        atomicExch(err, 1);
+        ok = false;
+      } else {
+        if (!cam_used[c]) cam_used[c] = 1;
+        if (!intr_used[g]) intr_used[g] = 1;
+      }
     }
-    atomicAdd(&counts[p], 1u);
-    cam_used[c] = 1;
-    intr_used[g] = 1;
+    const uint32_t before = __shfl_up_sync(0xffffffffu, p, 1);
+    const bool before_ok = __shfl_up_sync(0xffffffffu, (int)ok, 1) != 0;
+    const bool head = ok && (lane == 0 || !before_ok || before != p);
+    // the run ends at the next lane that starts another or has no observation
+    const uint32_t ends = __ballot_sync(0xffffffffu, head || !ok) & ~((2u << lane) - 1u);
+    if (head) atomicAdd(&counts[p], (uint32_t)((ends ? __ffs(ends) - 1 : 32) - lane));
   }
 }
 
@@ -361,7 +377,8 @@ __global__ void __launch_bounds__(256) k_linearize_max(Prob P, unsigned long lon
       // |v| as ordered bits; a non-finite term keeps the all-ones word (the
       // sums of its column become NaN)
       const double a = fabs(v);
-      atomicMax(p, finite_bits(a) ? (unsigned long long)__double_as_longlong(a) : ~0ull);
+      const unsigned long long b = finite_bits(a) ? (unsigned long long)__double_as_longlong(a) : ~0ull;
+      if (b > *p) atomicMax(p, b);  // (a stale word only costs the atomic)
     };
 #pragma unroll
     for (int j = 0; j < B; ++j) {
@@ -403,27 +420,80 @@ __global__ void __launch_bounds__(256) k_linearize(Prob P, double* __restrict__ 
   auto add = [](double* p, double v, int k) {
     atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)lin_fx(v, k));
   };
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < P.no; o += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  // few intrinsic groups: a warp adds its observations of a group first, as
+  // hundreds of thousands of atomics on a dozen words take turns (600k
+  // observations of 3 groups: 1.66 -> 0.29 ms)
+  const bool few = P.ni <= 64;
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; w0 < P.no; w0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t o = w0 + lane;
+    const bool valid = o < P.no;
     ObsJac<M, T> J;
     double cost;
-    obs_jacobian<M, T, false>(P, o, nullptr, nullptr, J, &cost);
+    uint32_t g = 0;
+    long long xn[B - 6], xg[B - 6];
+    if (valid) {
+      obs_jacobian<M, T, false>(P, o, nullptr, nullptr, J, &cost);
+      g = P.icam[o];
 #pragma unroll
-    for (int j = 0; j < B; ++j) {
-      if (J.col[j] < 0) continue;
-      const double a = J.Jc[0][j], b = J.Jc[1][j];
-      int en, eg;
-      lin_unpack(exp_c[J.col[j]], en, eg);
-      add(&cn_c[J.col[j]], a * a + b * b, en);
-      add(&g_c[J.col[j]], a * J.r[0] + b * J.r[1], eg);
+      for (int j = 0; j < B; ++j) {
+        if (j >= 6) xn[j - 6] = xg[j - 6] = 0;
+        if (J.col[j] < 0) continue;
+        const double a = J.Jc[0][j], b = J.Jc[1][j];
+        int en, eg;
+        lin_unpack(exp_c[J.col[j]], en, eg);
+        const long long vn = lin_fx(a * a + b * b, en), vg = lin_fx(a * J.r[0] + b * J.r[1], eg);
+        if (j >= 6) {
+          xn[j - 6] = vn;
+          xg[j - 6] = vg;
+        } else {
+          atomicAdd(reinterpret_cast<unsigned long long*>(&cn_c[J.col[j]]), (unsigned long long)vn);
+          atomicAdd(reinterpret_cast<unsigned long long*>(&g_c[J.col[j]]), (unsigned long long)vg);
+        }
+      }
+      const int64_t p = P.pt[o];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const double a = J.Jp[0][j], b = J.Jp[1][j];
+        int en, eg;
+        lin_unpack(exp_p[3 * p + j], en, eg);
+        add(&cn_p[3 * p + j], a * a + b * b, en);
+        add(&g_p[3 * p + j], a * J.r[0] + b * J.r[1], eg);
+      }
     }
-    const int64_t p = P.pt[o];
+    bool left = valid, sum = false;  // terms still to be added by this lane; they are a group's sum
+    while (few) {
+      const uint32_t todo = __ballot_sync(0xffffffffu, left && !sum);
+      if (!todo) break;
+      const int lead = __ffs(todo) - 1;
+      const uint32_t gl = __shfl_sync(0xffffffffu, g, lead);
+      const bool mine = left && !sum && g == gl;
+      if (__popc(__ballot_sync(0xffffffffu, mine)) < 4) break;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const double a = J.Jp[0][j], b = J.Jp[1][j];
-      int en, eg;
-      lin_unpack(exp_p[3 * p + j], en, eg);
-      add(&cn_p[3 * p + j], a * a + b * b, en);
-      add(&g_p[3 * p + j], a * J.r[0] + b * J.r[1], eg);
+      for (int j = 0; j < B - 6; ++j) {
+        long long sn = mine ? xn[j] : 0, sg = mine ? xg[j] : 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+          sn += __shfl_xor_sync(0xffffffffu, sn, d);
+          sg += __shfl_xor_sync(0xffffffffu, sg, d);
+        }
+        if (lane == lead) {
+          xn[j] = sn;
+          xg[j] = sg;
+        }
+      }
+      if (mine) {
+        sum = lane == lead;
+        left = sum;
+      }
+    }
+    if (left) {
+#pragma unroll
+      for (int j = 6; j < B; ++j) {
+        if (J.col[j] < 0) continue;
+        atomicAdd(reinterpret_cast<unsigned long long*>(&cn_c[J.col[j]]), (unsigned long long)xn[j - 6]);
+        atomicAdd(reinterpret_cast<unsigned long long*>(&g_c[J.col[j]]), (unsigned long long)xg[j - 6]);
+      }
     }
   }
 }
@@ -2572,11 +2642,16 @@ __global__ void k_cam_groups(const uint32_t* cam, const uint32_t* icam, int64_t 
                              int32_t* cam_group, uint32_t* group_cam, int* conflict, uint32_t* cam_hist) {
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < no; o += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t c = cam[o], g = icam[o];
-    const int32_t prev = atomicCAS(&cam_group[c], -1, (int32_t)g);
+    // (a plain load first: the words settle with their first observation, and
+    // a stale one only costs the exchange)
+    int32_t prev = cam_group[c];
+    if (prev != (int32_t)g) prev = atomicCAS(&cam_group[c], -1, (int32_t)g);
     if (prev != -1 && prev != (int32_t)g) atomicExch(conflict, 1);  // a camera of several groups
     if (intr_var[g]) {
-      const uint32_t pc = atomicCAS(&group_cam[g], 0xffffffffu, c);
-      if (pc != 0xffffffffu && pc != c) atomicExch(conflict + 1, 1);  // a free group of several cameras
+      if (group_cam[g] != c && !*(volatile int*)(conflict + 1)) {
+        const uint32_t pc = atomicCAS(&group_cam[g], 0xffffffffu, c);
+        if (pc != 0xffffffffu && pc != c) atomicExch(conflict + 1, 1);  // a free group of several cameras
+      }
     }
     atomicAdd(&cam_hist[c], 1u);
   }
