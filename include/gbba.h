@@ -76,8 +76,8 @@ typedef enum gbba_linear_solver {
   GBBA_SOLVER_DENSE_SCHUR = 1,     /* dense Cholesky of the reduced camera system S */
   GBBA_SOLVER_ITERATIVE_SCHUR = 2  /* block-Jacobi PCG on S; every free intrinsic group must belong to one
                                       camera (else GBBA_ERROR_NOT_SUPPORTED); the dense solver takes any
-                                      grouping (a free group shared by several cameras uses the point-major
-                                      Schur build, whose FP atomics are not bit-repeatable) */
+                                      grouping (cameras with several groups use the point-major Schur build,
+                                      whose FP atomics are not bit-repeatable) */
 } gbba_linear_solver;
 
 typedef enum gbba_precision {
@@ -86,10 +86,11 @@ typedef enum gbba_precision {
 } gbba_precision;
 
 /* How the dense path builds S.  AUTO takes the atomic-free camera-pair build
- * whenever every free intrinsic block belongs to one camera (S then splits
- * into camera-pair blocks) and the point-major build with atomic additions
- * otherwise; POINT_ATOMIC forces the latter (both give the same S up to the
- * order of the sums). */
+ * whenever every camera uses one intrinsic group (S then splits into
+ * camera-pair blocks, and into rows of the groups that cameras share: at most
+ * 64 free groups, about three per view of a point) and the point-major build
+ * with atomic additions otherwise; POINT_ATOMIC forces the latter (both give
+ * the same S up to the order of the sums). */
 typedef enum gbba_schur_build {
   GBBA_SCHUR_BUILD_AUTO = 0,
   GBBA_SCHUR_BUILD_POINT_ATOMIC = 1
