@@ -101,13 +101,13 @@ __global__ void __launch_bounds__(128) k_api_cam_lin(const double* __restrict__ 
 struct BackArgs {
   const double *ext, *lin, *intr, *pts, *obs;
   const uint32_t *cam, *icam, *pt;
-  int64_t no, nc, ni, ng;
+  int64_t no, nc, ni;
   int loss_type;
   double a;
   double *je, *jk, *jx;  // outputs, or null
   double* rc;            // corrected residuals of the stored blocks, or null
-  double* grad;          // fixed-point sums, or null
-  int* gexp;             // per gradient entry: exponent above its terms, then its scale
+  double* grad;          // largest |term| of each entry, then its fixed-point sum, or null
+  int* gexp;             // scale of each gradient entry
 };
 
 // The corrected blocks and residual of observation o.
@@ -143,6 +143,12 @@ __device__ __forceinline__ void back_blocks(const BackArgs& A, int64_t o, uint32
   }
 }
 
+// An observation's term of a gradient entry: the same rounding wherever it is
+// formed (the scale comes from the largest term as the first pass forms it).
+__device__ __forceinline__ double grad_term(double j0, double j1, double r0, double r1) {
+  return __fma_rn(j0, r0, __dmul_rn(j1, r1));
+}
+
 // W values per observation of a warp's 32 consecutive observations (`cnt` of
 // them) to out: through shared memory, so that the stores are consecutive.
 template <int W, typename T>
@@ -157,12 +163,13 @@ __device__ __forceinline__ void warp_store(double* __restrict__ out, int64_t o0,
 
 // Bound by the FP64 pipe (about 250 operations an observation) and by the 272
 // bytes written for it.  Before, every observation differentiated the rotation
-// again, its blocks left lane by lane, a pass in front found the exponents and
+// again, its blocks left lane by lane, a pass in front found the largest terms and
 // the gradient evaluated everything a third time: 300 cameras, 1M observations
-// 1673 -> 680 us for blocks, residuals and gradient (2.4x).
+// 1673 -> 740 us for blocks, residuals and gradient (2.3x; 666 us with scales
+// from the exponents of J and r alone, which left two to three bits of every
+// sum unused).
 // The blocks of every observation (32 consecutive ones per warp), and with a
-// gradient each entry's exponent bound: |J0 r0 + J1 r1| < 2^(max(e(J0) + e(r0),
-// e(J1) + e(r1)) + 1) from the exponents alone.
+// gradient the largest term of each of its entries.
 constexpr int kBackThreads = 128;
 template <int M, typename T>
 __global__ void __launch_bounds__(kBackThreads) k_backward(BackArgs A) {
@@ -179,15 +186,17 @@ __global__ void __launch_bounds__(kBackThreads) k_backward(BackArgs A) {
     double rc[2];
     back_blocks<M, T>(A, o, c, g, p, Je, Jk, Jx, rc);
     if (A.grad && lane < cnt) {
-      const int e0 = exp_above(rc[0]), e1 = exp_above(rc[1]);
-      auto bound = [&](int64_t idx, T j0, T j1) {
-        const int e = max(exp_above((double)j0) + e0, exp_above((double)j1) + e1) + 1;
-        int* q = A.gexp + idx;
-        if (*(volatile int*)q < e) atomicMax(q, e);  // it only grows: a stale value costs an atomic
+      // |term| as ordered bits; all ones for a non-finite one
+      auto largest = [&](int64_t idx, T j0, T j1) {
+        const double v = grad_term((double)j0, (double)j1, rc[0], rc[1]);
+        const unsigned long long b = (__double2hiint(v) & 0x7ff00000) == 0x7ff00000
+                                         ? ~0ull : (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+        unsigned long long* q = reinterpret_cast<unsigned long long*>(A.grad) + idx;
+        if (*(volatile unsigned long long*)q < b) atomicMax(q, b);  // it only grows: a stale value costs an atomic
       };
-      for (int j = 0; j < 6; ++j) bound(6 * (int64_t)c + j, Je[0][j], Je[1][j]);
-      for (int j = 0; j < K; ++j) bound(6 * A.nc + K * (int64_t)g + j, Jk[0][j], Jk[1][j]);
-      for (int j = 0; j < 3; ++j) bound(6 * A.nc + K * A.ni + 3 * (int64_t)p + j, Jx[0][j], Jx[1][j]);
+      for (int j = 0; j < 6; ++j) largest(6 * (int64_t)c + j, Je[0][j], Je[1][j]);
+      for (int j = 0; j < K; ++j) largest(6 * A.nc + K * (int64_t)g + j, Jk[0][j], Jk[1][j]);
+      for (int j = 0; j < 3; ++j) largest(6 * A.nc + K * A.ni + 3 * (int64_t)p + j, Jx[0][j], Jx[1][j]);
     }
     if (A.je) warp_store<12>(A.je, o0, cnt, &Je[0][0], sh);
     if (A.jk) warp_store<2 * K>(A.jk, o0, cnt, &Jk[0][0], sh);
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(kBackThreads) k_backward(BackArgs A) {
 }
 
 // The gradient's deterministic sums (see lin_fx): every entry's terms in fixed
-// point, scaled by its exponent bound.  kStored: from the blocks and residuals
+// point, scaled by its largest one.  kStored: from the blocks and residuals
 // that k_backward wrote (256 B an observation), else evaluated again.
 template <int M, typename T, bool kStored>
 __global__ void __launch_bounds__(256) k_backward_sum(BackArgs A) {
@@ -214,7 +223,7 @@ __global__ void __launch_bounds__(256) k_backward_sum(BackArgs A) {
       const double r0 = A.rc[2 * o], r1 = A.rc[2 * o + 1];
       auto block = [&](const double* __restrict__ J, int n, int64_t base) {
 #pragma unroll
-        for (int j = 0; j < n; ++j) put(base + j, J[j] * r0 + J[n + j] * r1);
+        for (int j = 0; j < n; ++j) put(base + j, grad_term(J[j], J[n + j], r0, r1));
       };
       block(A.je + 12 * o, 6, 6 * (int64_t)c);
       block(A.jk + 2 * K * o, K, 6 * A.nc + K * (int64_t)g);
@@ -223,19 +232,23 @@ __global__ void __launch_bounds__(256) k_backward_sum(BackArgs A) {
       T Je[2][6], Jk[2][K], Jx[2][3];
       double rc[2];
       back_blocks<M, T>(A, o, c, g, p, Je, Jk, Jx, rc);
-      for (int j = 0; j < 6; ++j) put(6 * (int64_t)c + j, (double)Je[0][j] * rc[0] + (double)Je[1][j] * rc[1]);
-      for (int j = 0; j < K; ++j) put(6 * A.nc + K * (int64_t)g + j, (double)Jk[0][j] * rc[0] + (double)Jk[1][j] * rc[1]);
-      for (int j = 0; j < 3; ++j)
-        put(6 * A.nc + K * A.ni + 3 * (int64_t)p + j, (double)Jx[0][j] * rc[0] + (double)Jx[1][j] * rc[1]);
+      auto term = [&](T j0, T j1) { return grad_term((double)j0, (double)j1, rc[0], rc[1]); };
+      for (int j = 0; j < 6; ++j) put(6 * (int64_t)c + j, term(Je[0][j], Je[1][j]));
+      for (int j = 0; j < K; ++j) put(6 * A.nc + K * (int64_t)g + j, term(Jk[0][j], Jk[1][j]));
+      for (int j = 0; j < 3; ++j) put(6 * A.nc + K * A.ni + 3 * (int64_t)p + j, term(Jx[0][j], Jx[1][j]));
     }
   }
 }
 
-// Between the gradient's passes: each entry's scale from its exponent bound;
-// after them: back to FP64 (NaN for an entry with a non-finite term).
-__global__ void k_grad_exp(int64_t n, double nobs, int* __restrict__ gexp) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    gexp[i] = lin_exp_of(gexp[i], nobs);
+// Between the gradient's passes: each entry's scale from its largest term, and
+// the entry cleared for the fixed-point sum; after them: back to FP64 (NaN for
+// an entry with a non-finite term).
+__global__ void k_grad_exp(int64_t n, double nobs, double* __restrict__ grad, int* __restrict__ gexp) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    unsigned long long* q = reinterpret_cast<unsigned long long*>(grad + i);
+    gexp[i] = lin_exp(*q, nobs);
+    *q = 0ull;
+  }
 }
 __global__ void k_grad_conv(int64_t n, double* __restrict__ grad, const int* __restrict__ gexp) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -598,7 +611,7 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
     const size_t bx = jac_point ? sizeof(double) * no * 6 : 0;
     const int64_t ng = 6 * nc + k * ni + 3 * np;
     const size_t bg = gradient ? sizeof(double) * ng : 0;
-    const size_t bgx = gradient ? sizeof(int) * ng : 0;  // the gradient entries' exponents
+    const size_t bgx = gradient ? sizeof(int) * ng : 0;  // the gradient entries' scale exponents
     const bool stored = be && bk && bx && bg;            // the gradient is summed from the stored blocks
     const size_t brc = stored ? sizeof(double) * 2 * no : 0;
     const size_t bl = fp32 ? 0 : sizeof(double) * kCamLin * nc;
@@ -622,13 +635,10 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
     A.lin = lin;
     A.ext = s.ext, A.intr = s.intr, A.pts = s.pts, A.obs = s.obs;
     A.cam = s.cam, A.icam = s.icam, A.pt = s.pt;
-    A.no = no, A.nc = nc, A.ni = ni, A.ng = ng;
+    A.no = no, A.nc = nc, A.ni = ni;
     A.loss_type = loss_type, A.a = loss_scale;
     cudaStream_t st = h->active;
-    if (A.grad) {
-      GBBA_CUDA(cudaMemsetAsync(A.grad, 0, bg, st));
-      GBBA_CUDA(cudaMemsetAsync(A.gexp, 0x80, bgx, st));  // below every exponent
-    }
+    if (A.grad) GBBA_CUDA(cudaMemsetAsync(A.grad, 0, bg, st));
     if (lin && nc > 0) {
       k_api_cam_lin<<<(unsigned)ceil_div(nc, 128), 128, 0, st>>>(s.ext, nc, lin);
       check_launch(h);
@@ -636,14 +646,14 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
     const int grid = std::max(1, std::min<int>((int)ceil_div(std::max<int64_t>(no, 1), 256), h->sm_count * 8));
     const unsigned gg = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ng, 256), 4096));
     auto run = [&](auto blocks, auto sum_stored, auto sum) {
-      // the blocks and, with a gradient, its entries' exponents; their scales;
+      // the blocks and, with a gradient, its entries' largest terms; their scales;
       // the fixed-point sums; back to FP64
       if (no > 0) {
         blocks<<<(unsigned)std::min<int64_t>(ceil_div(no, kBackThreads), (int64_t)h->sm_count * 16), kBackThreads, 0, st>>>(A);
         check_launch(h);
       }
       if (!A.grad) return;
-      k_grad_exp<<<gg, 256, 0, st>>>(ng, (double)std::max<int64_t>(1, no), A.gexp);
+      k_grad_exp<<<gg, 256, 0, st>>>(ng, (double)std::max<int64_t>(1, no), A.grad, A.gexp);
       check_launch(h);
       if (no > 0) {
         if (stored) sum_stored<<<grid, 256, 0, st>>>(A);

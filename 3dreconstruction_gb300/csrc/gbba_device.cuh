@@ -366,22 +366,6 @@ __device__ __forceinline__ int lin_exp(unsigned long long mbits, double n) {
   frexp(m * n, &e);  // m n < 2^e
   return 62 - e;
 }
-// The same from an exponent e with |term| < 2^e for every term (above 1020:
-// non-finite; below every exponent: no term).
-__device__ __forceinline__ int lin_exp_of(int e, double n) {
-  if (e > 1020) return kFxNonFinite;
-  if (e < -4096) return 0;
-  int en;
-  frexp(n, &en);  // n < 2^en
-  return 62 - e - en;
-}
-// Exponent of a double, |v| < 2^e (no FP64 operation); for infinities and NaN
-// so large that the sum with any other stays above 1020 (their product with a
-// small value or a zero is not finite either).
-__device__ __forceinline__ int exp_above(double v) {
-  const int ex = (int)((__double2hiint(v) >> 20) & 0x7ff);
-  return ex == 0x7ff ? 1 << 20 : ex - 1022;
-}
 // v 2^k rounded to an integer with integer operations (|v| 2^k < 2^62 by
 // the choice of k); any rounding rule serves, the sum is exact.
 __device__ __forceinline__ long long lin_fx(double v, int k) {
