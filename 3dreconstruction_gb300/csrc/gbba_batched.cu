@@ -1428,9 +1428,11 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     k_batch_index<<<dim3(np_, (unsigned)std::min<int64_t>(ceil_div(most, 4096), 4096)), 256, 0, st>>>(
         in.probs, in.cam, in.icam, in.pt, in.used, in.used + tc, in.counts, in.err);
     check_launch(h);
-    k_batch_views<<<(unsigned)std::min<int64_t>(ceil_div(tx, 256), h->sm_count * 8), 256, 0, st>>>(in.counts, tx,
-                                                                                                   in.err + np_);
-    check_launch(h);
+    if (tx > 0) {  // (observations of no point at all are refused below)
+      k_batch_views<<<(unsigned)std::min<int64_t>(ceil_div(tx, 256), h->sm_count * 8), 256, 0, st>>>(in.counts, tx,
+                                                                                                     in.err + np_);
+      check_launch(h);
+    }
   }
   std::vector<uint32_t> err(np_ + 1);
   std::vector<uint8_t> used(tc + tg);
