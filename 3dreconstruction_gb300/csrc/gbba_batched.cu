@@ -1393,6 +1393,12 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     if (mem == GBBA_MEMORY_HOST) std::memcpy(dst, src, bytes);
     else GBBA_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
   };
+  // Device arrays may come from work that the caller has just queued on the
+  // default stream, which the call's own stream does not wait for by itself.
+  if (mem == GBBA_MEMORY_DEVICE) {
+    GBBA_CUDA(cudaEventRecord(h->ev_main, cudaStreamLegacy));
+    GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_main, 0));
+  }
   // per-window flags and constants
   Planner ps;
   auto stage = [&](auto& A) {
