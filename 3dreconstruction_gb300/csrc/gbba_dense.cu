@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "gbba_internal.h"
+#include "gbba_pivot.cuh"
 #include "gbba_umma.cuh"
 
 namespace gbba {
@@ -734,35 +735,6 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ S, int64
 constexpr int kDigits = 8;
 constexpr int kDigitTile = 64 * 64;                            // one digit of a 64 x 64 tile (8 KB of FP16)
 constexpr size_t kTileDigitBytes = (size_t)kDigits * kDigitTile * 2;
-
-// 1 / d from the hardware's approximate reciprocal r: with e = 1 - d r, the
-// next terms of the geometric series 1 / d = r (1 + e + e^2 + ...) (Newton's
-// iteration of third order).
-__device__ __forceinline__ double rcp_series(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-// s = sqrt(d) and r = 1 / s: two of Newton's steps y += y (1 - d y^2) / 2 from
-// the hardware's approximation of 1 / sqrt(d), then s = d y and r = y with a
-// last step each, so that s r = 1 to rounding.
-__device__ __forceinline__ void sqrt_newton(double d, double& s, double& r) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double e = fma(-d * y, y, 1.0);
-    y = fma(0.5 * y, e, y);
-  }
-  s = d * y;
-  s = fma(0.5 * y, fma(-s, s, d), s);
-  r = fma(y, fma(-s, y, 1.0), y);
-}
-__device__ __forceinline__ bool positive_finite(double d) {  // on the bits: FP64 comparisons run on the FP64 pipe
-  const unsigned hi = (unsigned)__double2hiint(d);
-  return hi < 0x7ff00000u && (hi | (unsigned)__double2loint(d)) != 0u;
-}
 
 // Panel kb: [L_kk; L_ik] of the diagonal tile and of this CTA's rows below it,
 // y_kb = L_kk^-1 b_kb, b_i -= L_ik y_kb and the digits of the rows.  L_kk with
