@@ -2620,13 +2620,18 @@ __global__ void k_convert(const T* a, U2* b, int64_t n) {
 
 // ---------------------------------------------------------------- pair-list setup kernels
 // Per point: number of ordered observation pairs (a, b) with cam(a) >= cam(b).
-__global__ void k_pair_count(const uint32_t* pt_off, const uint32_t* cam, int64_t np, uint32_t* cnt) {
+// (*total: their number, which may exceed what the 32-bit offsets can hold)
+__global__ void k_pair_count(const uint32_t* pt_off, const uint32_t* cam, int64_t np, uint32_t* cnt,
+                             unsigned long long* total) {
+  unsigned long long all = 0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t n = 0;
+    unsigned long long n = 0;
     for (uint32_t a = pt_off[p]; a < pt_off[p + 1]; ++a)
       for (uint32_t b = pt_off[p]; b < pt_off[p + 1]; ++b) n += cam[a] >= cam[b];
-    cnt[p] = n;
+    cnt[p] = (uint32_t)n;
+    all += n;
   }
+  if (all) atomicAdd(total, all);
 }
 __global__ void k_pair_write(const uint32_t* pt_off, const uint32_t* cam, int64_t np, int64_t nc, const uint32_t* pair_off,
                              unsigned long long* pairs, uint32_t* keys, uint32_t* hist) {
@@ -3541,7 +3546,7 @@ static void setup(gbba_handle* h, const gbba_problem* P, const gbba_options* o, 
 static void setup_atomic_path(gbba_handle* h, Solve& s, size_t tsize) {
   GBBA_REQUIRE(s.dense, GBBA_ERROR_NOT_SUPPORTED,
                "the iterative Schur solver needs every free intrinsic block to belong to one camera");
-  s.pair_path = false;
+  s.pair_path = s.shared = false;
   Arena& A = h->pair_arena;
   const size_t w = (size_t)s.no * (6 + s.k) * 3 * tsize;
   A.reset();
@@ -3550,7 +3555,24 @@ static void setup_atomic_path(gbba_handle* h, Solve& s, size_t tsize) {
   s.What = A.take<char>(w);
 }
 
+// Pairs that the camera-pair list can hold (its sort counts them in an int).
+constexpr unsigned long long kMaxPairs = 0x7fffffffull;
+
+static void setup_pair_path(gbba_handle* h, Solve& s, size_t tsize);
 static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
+  try {
+    setup_pair_path(h, s, tsize);
+  } catch (const Error& e) {
+    // Shared groups do with the point-major build, which needs less: two
+    // thirds of the records and no pair list, group blocks or work items.
+    if (e.status != GBBA_ERROR_OUT_OF_MEMORY || !s.shared) throw;
+    cudaGetLastError();  // the failed allocation's
+    h->item_arena.release();
+    setup_atomic_path(h, s, tsize);
+  }
+}
+
+static void setup_pair_path(gbba_handle* h, Solve& s, size_t tsize) {
   s.pair_path = false;
   const int64_t nc = s.nc, ni = s.ni, np = s.np, no = s.no;
   const bool want_pairs = s.dense;
@@ -3578,6 +3600,7 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     p1.take<uint32_t>(ceil_div(std::max(np, nk) + 1, 1024) + 1);
     p1.take<uint32_t>(np + 1);
     p1.take<uint32_t>(np + 1);
+    p1.take<unsigned long long>(1);
     p1.take<char>((size_t)no * (s.dense ? 9 * B + 8 : 2 * B + 16) * tsize);
     // PCG vectors (x, r, z, p, q, b), point temporaries, camera blocks
     p1.take<double>(6 * n_pcg);
@@ -3608,6 +3631,7 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     uint32_t* chunks = A.take<uint32_t>(ceil_div(std::max(np, nk) + 1, 1024) + 1);
     uint32_t* pcnt = A.take<uint32_t>(np + 1);
     uint32_t* pair_off = A.take<uint32_t>(np + 1);
+    unsigned long long* pair_total = A.take<unsigned long long>(1);
     s.rec = A.take<char>((size_t)no * (s.dense ? 9 * B + 8 : 2 * B + 16) * tsize);
     s.pcg_x = A.take<double>(n_pcg);
     s.pcg_r = A.take<double>(n_pcg);
@@ -3635,22 +3659,25 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     GBBA_CUDA(cudaMemsetAsync(conflict, 0, sizeof(int) * 2, st));
     GBBA_CUDA(cudaMemsetAsync(cam_hist, 0, sizeof(uint32_t) * (nc + 1), st));
     GBBA_CUDA(cudaMemsetAsync(cam_fill, 0, sizeof(uint32_t) * (nc + 1), st));
+    GBBA_CUDA(cudaMemsetAsync(pair_total, 0, sizeof(unsigned long long), st));
     const int grid = s.nb_obs;
     k_cam_groups<<<grid, 256, 0, st>>>(s.cam, s.icam, no, s.intr_var, s.cam_group, group_cam, conflict, cam_hist);
     check_launch(h);
-    k_pair_count<<<std::max(1, (int)std::min<int64_t>(ceil_div(np, 128), h->sm_count * 16)), 128, 0, st>>>(s.pt_off, s.cam, np, pcnt);
+    k_pair_count<<<std::max(1, (int)std::min<int64_t>(ceil_div(np, 128), h->sm_count * 16)), 128, 0, st>>>(s.pt_off, s.cam, np, pcnt,
+                                                                                                            pair_total);
     check_launch(h);
     scan_offsets(h, pcnt, pair_off, np, chunks, st);
     int hconf[2] = {0, 0};
-    uint32_t total = 0;
+    unsigned long long all_pairs = 0;
     GBBA_CUDA(cudaMemcpyAsync(hconf, conflict, sizeof(hconf), cudaMemcpyDeviceToHost, st));
-    GBBA_CUDA(cudaMemcpyAsync(&total, pair_off + np, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    GBBA_CUDA(cudaMemcpyAsync(&all_pairs, pair_total, sizeof(all_pairs), cudaMemcpyDeviceToHost, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
     // Shared groups: G and H of every point and group, at most twice the
     // records (6 K np ng values against (9 B + 8) no), and a mask of 64 groups.
-    // Beyond that, and for cameras with several groups, the point-major build.
+    // Beyond that, for cameras with several groups, and for more pairs than the
+    // list can hold, the point-major build.
     s.shared = hconf[1] != 0;
-    if (hconf[0] ||
+    if (hconf[0] || (want_pairs && all_pairs > kMaxPairs) ||
         (s.shared && (!s.dense || s.n_free > 64 || (int64_t)6 * s.k * np * s.n_free > 2 * no * (9 * B + 8)))) {
       setup_atomic_path(h, s, tsize);
       return;
@@ -3662,7 +3689,7 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
     else s.block_group = s.cam_group;
     s.bb = ext_only ? 6 : B;
     Planner p2;
-    if (!want_pairs) total = 0;
+    const uint32_t total = want_pairs ? (uint32_t)all_pairs : 0;
     size_t pair_sort_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, pair_sort_bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
                                     (const unsigned long long*)nullptr, (unsigned long long*)nullptr, (int)total, 0,
