@@ -262,8 +262,44 @@ struct Staged {
   const uint32_t *cam, *icam, *pt;
 };
 
-// Make the problem's arrays device-resident (copies for host memory, the
-// caller's own arrays otherwise) and check indices.
+// An array of the call in the caller's memory.
+struct Span {
+  const void* p;
+  size_t bytes;
+  bool aligned(size_t to) const { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; }
+  bool overlaps(const Span& o) const {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(o.p);
+    return bytes && o.bytes && a < b + o.bytes && b < a + bytes;
+  }
+};
+struct Inputs {
+  Span a[7];  // extrinsics, intrinsics, points, observations, the three indices
+};
+static Inputs input_spans(const gbba_problem* P) {
+  const size_t no = P->num_observations;
+  return {{{P->extrinsics, sizeof(double) * 6 * P->num_cameras},
+           {P->intrinsics, sizeof(double) * model_k(P->camera_model) * P->num_intrinsics},
+           {P->points, sizeof(double) * 3 * P->num_points},
+           {P->observations, sizeof(double) * 2 * no},
+           {P->camera_index, sizeof(uint32_t) * no},
+           {P->intrinsic_index, sizeof(uint32_t) * no},
+           {P->point_index, sizeof(uint32_t) * no}}};
+}
+// Whether the kernels write output `o` where the caller wants it: an aligned
+// array in device memory apart from everything else that the call reads or
+// writes.  Other outputs are staged and copied out at the end.
+static bool in_place(const gbba_problem* P, const Span& o, const Span* others = nullptr, int n = 0) {
+  if (P->memory == GBBA_MEMORY_HOST || !o.aligned(sizeof(double))) return false;
+  for (const Span& i : input_spans(P).a)
+    if (o.overlaps(i)) return false;
+  for (int i = 0; i < n; ++i)
+    if (&others[i] != &o && o.overlaps(others[i])) return false;
+  return true;
+}
+
+// Make the problem's arrays device-resident and check indices: the caller's
+// own arrays in device memory that the kernels can read (aligned for their
+// type), else copies.
 static Staged stage(gbba_handle* h, const gbba_problem* P, size_t extra_bytes, char** extra) {
   const int64_t no = P->num_observations, nc = P->num_cameras, ni = P->num_intrinsics, np = P->num_points;
   const int k = model_k(P->camera_model);
@@ -273,26 +309,28 @@ static Staged stage(gbba_handle* h, const gbba_problem* P, size_t extra_bytes, c
   pl.take<double>(k * ni);
   pl.take<double>(3 * np);
   pl.take<double>(2 * no);
-  pl.take<uint32_t>(3 * no);
+  for (int i = 0; i < 3; ++i) pl.take<uint32_t>(no);
   pl.take<int>(1);
   pl.take<char>(extra_bytes);
   h->arena.reset();
   h->arena.reserve(pl.used + 4096);
   Staged s;
   const bool host = P->memory == GBBA_MEMORY_HOST;
-  auto put = [&](const void* src, size_t bytes) -> const void* {
-    if (!host) return src;
-    void* d = h->arena.take<char>(bytes);
-    if (bytes) GBBA_CUDA(cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, st));
+  auto put = [&](const Span& src, size_t align) -> const void* {
+    if (!host && src.aligned(align)) return src.p;
+    void* d = h->arena.take<char>(src.bytes);
+    if (src.bytes)
+      GBBA_CUDA(cudaMemcpyAsync(d, src.p, src.bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
     return d;
   };
-  s.ext = (const double*)put(P->extrinsics, sizeof(double) * 6 * nc);
-  s.intr = (const double*)put(P->intrinsics, sizeof(double) * k * ni);
-  s.pts = (const double*)put(P->points, sizeof(double) * 3 * np);
-  s.obs = (const double*)put(P->observations, sizeof(double) * 2 * no);
-  s.cam = (const uint32_t*)put(P->camera_index, sizeof(uint32_t) * no);
-  s.icam = (const uint32_t*)put(P->intrinsic_index, sizeof(uint32_t) * no);
-  s.pt = (const uint32_t*)put(P->point_index, sizeof(uint32_t) * no);
+  const Inputs in = input_spans(P);
+  s.ext = (const double*)put(in.a[0], sizeof(double));
+  s.intr = (const double*)put(in.a[1], sizeof(double));
+  s.pts = (const double*)put(in.a[2], sizeof(double));
+  s.obs = (const double*)put(in.a[3], sizeof(double));
+  s.cam = (const uint32_t*)put(in.a[4], sizeof(uint32_t));
+  s.icam = (const uint32_t*)put(in.a[5], sizeof(uint32_t));
+  s.pt = (const uint32_t*)put(in.a[6], sizeof(uint32_t));
   int* err = h->arena.take<int>(1);
   *extra = h->arena.take<char>(extra_bytes);
   GBBA_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
@@ -572,11 +610,11 @@ gbba_status gbba_project_forward(gbba_handle* h, const gbba_problem* P, int32_t 
   return guarded(h, nullptr, [&]() {
     const int64_t no = P->num_observations;
     const int grid = std::max(1, std::min<int>((int)ceil_div(std::max<int64_t>(no, 1), 256), h->sm_count * 8));
-    const bool host = P->memory == GBBA_MEMORY_HOST;
-    const size_t res_bytes = residuals && host ? sizeof(double) * 2 * no : 0;  // device memory: written in place
+    const Span out{residuals, residuals ? sizeof(double) * 2 * no : 0};
+    const size_t res_bytes = in_place(P, out) ? 0 : out.bytes;
     char* extra;
     Staged s = stage(h, P, res_bytes + sizeof(double) * grid, &extra);
-    double* dres = !residuals ? nullptr : host ? (double*)extra : residuals;
+    double* dres = !residuals ? nullptr : res_bytes ? (double*)extra : residuals;
     double* part = (double*)(extra + res_bytes);
     cudaStream_t st = h->active;
     switch (P->camera_model) {
@@ -587,7 +625,7 @@ gbba_status gbba_project_forward(gbba_handle* h, const gbba_problem* P, int32_t 
     check_launch(h);
     std::vector<double> hp(grid);
     GBBA_CUDA(cudaMemcpyAsync(hp.data(), part, sizeof(double) * grid, cudaMemcpyDeviceToHost, st));
-    if (res_bytes) GBBA_CUDA(cudaMemcpyAsync(residuals, dres, res_bytes, cudaMemcpyDeviceToHost, st));
+    if (res_bytes) GBBA_CUDA(cudaMemcpyAsync(residuals, dres, res_bytes, cudaMemcpyDefault, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
     double c = 0.0;
     for (double v : hp) c += v;
@@ -604,8 +642,6 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
   return guarded(h, nullptr, [&]() {
     const int64_t no = P->num_observations, nc = P->num_cameras, ni = P->num_intrinsics, np = P->num_points;
     const int k = model_k(P->camera_model);
-    // outputs: the caller's arrays in device memory, else staged ones
-    const bool host = P->memory == GBBA_MEMORY_HOST;
     const size_t be = jac_extrinsic ? sizeof(double) * no * 12 : 0;
     const size_t bk = jac_intrinsic ? sizeof(double) * no * 2 * k : 0;
     const size_t bx = jac_point ? sizeof(double) * no * 6 : 0;
@@ -616,19 +652,23 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
     const size_t brc = stored ? sizeof(double) * 2 * no : 0;
     const size_t bl = fp32 ? 0 : sizeof(double) * kCamLin * nc;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    auto own = [&](size_t b) { return host ? al(b) : 0; };
+    // outputs: the caller's arrays where they can be written, else staged ones
+    double* const user[4] = {jac_extrinsic, jac_intrinsic, jac_point, gradient};
+    const Span outs[4] = {{jac_extrinsic, be}, {jac_intrinsic, bk}, {jac_point, bx}, {gradient, bg}};
+    size_t own[4];  // bytes staged
+    for (int i = 0; i < 4; ++i) own[i] = in_place(P, outs[i], outs, 4) ? 0 : al(outs[i].bytes);
     char* extra;
-    Staged s = stage(h, P, own(be) + own(bk) + own(bx) + own(bg) + al(bgx) + al(brc) + al(bl), &extra);
-    auto out = [&](double* user, size_t b) {
-      double* d = !b ? nullptr : host ? (double*)extra : user;
-      extra += own(b);
+    Staged s = stage(h, P, own[0] + own[1] + own[2] + own[3] + al(bgx) + al(brc) + al(bl), &extra);
+    auto out = [&](int i) {
+      double* d = !outs[i].bytes ? nullptr : own[i] ? (double*)extra : user[i];
+      extra += own[i];
       return d;
     };
     BackArgs A;
-    A.je = out(jac_extrinsic, be);
-    A.jk = out(jac_intrinsic, bk);
-    A.jx = out(jac_point, bx);
-    A.grad = out(gradient, bg);
+    A.je = out(0);
+    A.jk = out(1);
+    A.jx = out(2);
+    A.grad = out(3);
     A.gexp = bgx ? (int*)extra : nullptr;
     A.rc = brc ? (double*)(extra + al(bgx)) : nullptr;
     double* lin = bl ? (double*)(extra + al(bgx) + al(brc)) : nullptr;
@@ -673,12 +713,9 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
       case kRadialK3: model(std::integral_constant<int, kRadialK3>()); break;
       default: model(std::integral_constant<int, kBrownT2>()); break;
     }
-    if (host) {
-      if (be) GBBA_CUDA(cudaMemcpyAsync(jac_extrinsic, A.je, be, cudaMemcpyDeviceToHost, st));
-      if (bk) GBBA_CUDA(cudaMemcpyAsync(jac_intrinsic, A.jk, bk, cudaMemcpyDeviceToHost, st));
-      if (bx) GBBA_CUDA(cudaMemcpyAsync(jac_point, A.jx, bx, cudaMemcpyDeviceToHost, st));
-      if (bg) GBBA_CUDA(cudaMemcpyAsync(gradient, A.grad, bg, cudaMemcpyDeviceToHost, st));
-    }
+    const double* const written[4] = {A.je, A.jk, A.jx, A.grad};
+    for (int i = 0; i < 4; ++i)
+      if (own[i]) GBBA_CUDA(cudaMemcpyAsync(user[i], written[i], outs[i].bytes, cudaMemcpyDefault, st));
     GBBA_CUDA(cudaStreamSynchronize(st));
     return GBBA_SUCCESS;
   });
