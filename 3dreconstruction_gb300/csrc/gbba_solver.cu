@@ -3949,9 +3949,9 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   const bool many = !kPose && s.no >= 16384;
   // camera data of the current parameters: poses (mixed path) or linearisation data (FP64 path)
   auto camera_data = [&]() {
-    if (s.nc == 0) return;
+    if (s.nc == 0 || !(kPose || many)) return;
     if (kPose) k_cam_pose<<<nb_cam_pose, 128, 0, st>>>(s.ext, s.nc, s.pose);
-    else if (many) k_cam_lin<<<(unsigned)ceil_div(s.nc, 64), 64, 0, st>>>(s.ext, s.nc, s.lin);
+    else k_cam_lin<<<(unsigned)ceil_div(s.nc, 64), 64, 0, st>>>(s.ext, s.nc, s.lin);
     check_launch(h);
   };
   auto to_float = [&](const double* src, float* dst, int64_t n) {
