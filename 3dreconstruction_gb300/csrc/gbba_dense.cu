@@ -729,9 +729,14 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ S, int64
 // |d_p| <= 128.  The digit products of equal weight p + q = g, g = 0..7, are
 // summed in one FP32 accumulator each: at most 8 products of 64 terms of at
 // most 2^14, so every partial sum is an integer of at most 2^23, exact in
-// FP32.  The eight sums make a 62-bit integer with integer arithmetic; what is
-// left out is about 2^-59 max_k |l_ik| max_k |l_jk| per panel, less than the
-// rounding of 64 FP64 FMAs.
+// FP32.  The eight sums make a 62-bit integer with integer arithmetic.  Left out
+// are the products of weight 8 and more, seven pairs of digits of 64 terms of
+// at most 2^14 each: at most 2^-53.2 max_k |l_ik| max_k |l_jk| a panel, and about
+// 2^-59 of it when the digits' signs are random.  The two maxima are at most
+// sqrt(S_ii S_jj), so normwise this is within the rounding of a Cholesky
+// factorisation in FP64; an entry whose rows have their large values in
+// different columns keeps that absolute error, where an FMA would round each
+// of its small products relative to itself.
 constexpr int kDigits = 8;
 constexpr int kDigitTile = 64 * 64;                            // one digit of a 64 x 64 tile (8 KB of FP16)
 constexpr size_t kTileDigitBytes = (size_t)kDigits * kDigitTile * 2;
@@ -1237,7 +1242,7 @@ void dense_cholesky_prepare() {
 
 // Launch on the panel chain at the device's greatest stream priority (the
 // attribute is kept when the launch is captured into a graph), so that the
-// one-CTA diagonal factor is scheduled ahead of the trailing update's CTAs.
+// panel's CTAs are scheduled ahead of the trailing update's.
 //
 // With pdl the launch may begin while the previous kernel on the stream is
 // still running (programmatic dependent launch): the kernel must execute
@@ -1357,9 +1362,11 @@ static void dense_cholesky_solve_fp64(gbba_handle* h, double* S, int64_t n, int6
   }
   if (side_pending) GBBA_CUDA(cudaStreamWaitEvent(st, h->ev_side, 0));
   // The inverses of all tiles cost 27 us once, substitution by 16-column blocks
-  // about 2 us more in each step of the chain of block rows: one tile (two
-  // cameras, 20 iterations) 4.93 -> 4.62 ms a solve; the sides meet at some 12
-  // tiles.
+  // about half a microsecond more in each step of the chain of block rows.  10
+  // iterations with the blocks and with the inverses: 1 tile 2.93 and 3.17 ms, 4
+  // tiles 5.29 and 5.48, 8 tiles 8.07 and 8.22, 12 tiles 11.96 and 12.11, 20 tiles
+  // 18.31 and 18.45; by that slope the sides meet at some 45 tiles.  The line is
+  // short of it: larger systems keep the rounding of the inverses.
   const bool blocks = nb <= 8;
   if (!blocks) {
     k_tile_inverse<<<(unsigned)nb, 256, kTileInverseSmem, st>>>(Linv_all);

@@ -443,8 +443,11 @@ __global__ void __launch_bounds__(256) k_linearize(Prob P, double* __restrict__ 
   };
   const int lane = threadIdx.x & 31;
   // few intrinsic groups: a warp adds its observations of a group first, as
-  // hundreds of thousands of atomics on a dozen words take turns (600k
-  // observations of 3 groups: 1.66 -> 0.29 ms)
+  // hundreds of thousands of atomics on a dozen words take turns.  600k
+  // observations, by atomics and by warp sums: 1 group 1.63 and 0.28 ms, 3
+  // groups 1.65 and 0.29, 8 groups 1.49 and 1.07, 16 groups 1.43 and 1.37; from
+  // 32 groups on a warp holds less than four of any and both are the same (32
+  // groups 0.81 and 0.80, 64 0.53, 300 0.28)
   const bool few = P.ni <= 64;
   for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; w0 < P.no; w0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t o = w0 + lane;
@@ -1272,8 +1275,9 @@ __device__ __forceinline__ void write_block(uint32_t ca, uint32_t cb, const T* a
 
 // Register tiling of one B x B camera-pair block over a warp: lane t of a
 // group owns the 3x3 output tile (ti, tj) = (t / TPD, t % TPD).  When the
-// block needs at most 16 tiles the warp splits into two groups of 16 lanes
-// that take alternate pairs (their sums are added in group order at the end).
+// block needs at most 16 tiles the warp splits into two groups of 16 lanes, at
+// most 4 tiles into eight groups of 4, that take pairs in turn (their sums are
+// added in a fixed order at the end).
 // Staged operands are padded so that a tile's three rows are 16-byte loads:
 // W V^-1 and W as TPD groups of 12 values (3 rows x 3 + 3 padding), Jc as
 // 2 rows x TPD groups of 4 values (3 + 1 padding).
@@ -3539,10 +3543,8 @@ static void setup(gbba_handle* h, const gbba_problem* P, const gbba_options* o, 
 }
 
 
-// Pair list and camera CSR of the atomic-free Schur build.  Applies when the
-// dense solver is used, every free intrinsic block is private to one camera
-// and every camera uses one intrinsic group; otherwise the point-major kernel
-// with atomics is used.
+// The point-major build with atomics, for what the camera-pair list does not
+// cover or hold (setup_pair_path).
 static void setup_atomic_path(gbba_handle* h, Solve& s, size_t tsize) {
   GBBA_REQUIRE(s.dense, GBBA_ERROR_NOT_SUPPORTED,
                "the iterative Schur solver needs every free intrinsic block to belong to one camera");
@@ -3572,6 +3574,8 @@ static void setup_pairs(gbba_handle* h, Solve& s, size_t tsize) {
   }
 }
 
+// Pair list and camera CSR of the atomic-free Schur build (the iterative path:
+// the CSR alone), for cameras of one intrinsic group each.
 static void setup_pair_path(gbba_handle* h, Solve& s, size_t tsize) {
   s.pair_path = false;
   const int64_t nc = s.nc, ni = s.ni, np = s.np, no = s.no;
@@ -3942,10 +3946,14 @@ static gbba_status run_lm(Solve& s, const gbba_options* o, gbba_summary* sum) {
   // s.pose for the current parameters, s.pose2 for the evaluated ones.
   constexpr bool kPose = sizeof(T) == 4;
   const unsigned nb_cam_pose = (unsigned)std::max<int64_t>(1, ceil_div(s.nc, 128));
-  // The FP64 path shares per-camera terms from 16384 observations on, where a
-  // launch for them (5 us) costs less than the Rodrigues terms of every
-  // observation (about 90 FP64 operations a cost, 300 a Jacobian); at 800
-  // observations both ways measured the same.
+  // The FP64 path shares per-camera terms from 16384 observations on: a launch
+  // for them (5 us) against the Rodrigues terms of every observation (about 90
+  // FP64 operations a cost, 300 a Jacobian).  Time does not set the line: 10
+  // iterations with the per-camera terms and without take 2.59 and 2.62 ms at
+  // 1,150 observations, 3.43 and 3.43 at 3,900, 4.72 and 4.75 at 8,000, 7.48 and
+  // 7.53 at 16,000, 13.56 and 13.64 at 32,000.  Below it a solve keeps the
+  // rounding of the Rodrigues form, since two cameras with a free scale carry
+  // any other rounding along the gauge into their last eight digits.
   const bool many = !kPose && s.no >= 16384;
   // camera data of the current parameters: poses (mixed path) or linearisation data (FP64 path)
   auto camera_data = [&]() {

@@ -88,9 +88,11 @@ typedef enum gbba_precision {
 /* How the dense path builds S.  AUTO takes the atomic-free camera-pair build
  * whenever every camera uses one intrinsic group (S then splits into
  * camera-pair blocks, and into rows of the groups that cameras share: at most
- * 64 free groups, about three per view of a point) and the point-major build
- * with atomic additions otherwise; POINT_ATOMIC forces the latter (both give
- * the same S up to the order of the sums). */
+ * 64 free groups, about three per view of a point), as long as the pairs of
+ * observations of a same point number at most 2^31 - 1 and, with shared groups,
+ * their list fits the device memory; otherwise the point-major build with
+ * atomic additions.  POINT_ATOMIC forces the latter (both give the same S up to
+ * the order of the sums). */
 typedef enum gbba_schur_build {
   GBBA_SCHUR_BUILD_AUTO = 0,
   GBBA_SCHUR_BUILD_POINT_ATOMIC = 1
