@@ -2629,9 +2629,13 @@ __global__ void k_pair_count(const uint32_t* pt_off, const uint32_t* cam, int64_
                              unsigned long long* total) {
   unsigned long long all = 0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t begin = pt_off[p], end = pt_off[p + 1];
     unsigned long long n = 0;
-    for (uint32_t a = pt_off[p]; a < pt_off[p + 1]; ++a)
-      for (uint32_t b = pt_off[p]; b < pt_off[p + 1]; ++b) n += cam[a] >= cam[b];
+    for (uint32_t a = begin; a < end; ++a) {
+      uint32_t m = 0;
+      for (uint32_t b = begin; b < end; ++b) m += cam[a] >= cam[b];
+      n += m;
+    }
     cnt[p] = (uint32_t)n;
     all += n;
   }
