@@ -13,6 +13,8 @@ namespace gbba {
 gbba_status solve_impl(gbba_handle* h, const gbba_problem* P, const gbba_options* o, gbba_summary* sum);
 gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_t n, const gbba_options* o,
                                gbba_summary* sums);
+// FP64 linearisation data of every camera (the solver's).
+__global__ void k_cam_lin(const double* __restrict__ ext, int64_t nc, double* __restrict__ lin);
 
 static int model_k(int m) { return m == kPinholeF ? 1 : m == kRadialK3 ? 6 : 8; }
 
@@ -80,16 +82,6 @@ __global__ void __launch_bounds__(256) k_forward(const double* ext, const double
     for (int w = 0; w < 8; ++w) s += sh[w];
     part[blockIdx.x] = s;
   }
-}
-
-// FP64 linearisation data of every camera (residual_lin).
-__global__ void __launch_bounds__(128) k_api_cam_lin(const double* __restrict__ ext, int64_t nc, double* __restrict__ lin) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  double E[6], L[kCamLin];
-  for (int i = 0; i < 6; ++i) E[i] = ext[6 * c + i];
-  cam_lin(E, L);
-  for (int i = 0; i < kCamLin; ++i) lin[kCamLin * c + i] = L[i];
 }
 
 // Jacobian blocks and gradient of the robustified residual.  T = double is
@@ -680,7 +672,7 @@ static gbba_status project_backward(gbba_handle* h, const gbba_problem* P, int32
     cudaStream_t st = h->active;
     if (A.grad) GBBA_CUDA(cudaMemsetAsync(A.grad, 0, bg, st));
     if (lin && nc > 0) {
-      k_api_cam_lin<<<(unsigned)ceil_div(nc, 128), 128, 0, st>>>(s.ext, nc, lin);
+      k_cam_lin<<<(unsigned)ceil_div(nc, 64), 64, 0, st>>>(s.ext, nc, lin);
       check_launch(h);
     }
     const int grid = std::max(1, std::min<int>((int)ceil_div(std::max<int64_t>(no, 1), 256), h->sm_count * 8));
