@@ -1503,10 +1503,9 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     clustered = (int)(std::stable_partition(order.begin(), order.end(), [&](uint32_t i) { return load(i) > line; }) -
                       order.begin());
   }
-  const int64_t total_ctas = (int64_t)clustered * ctas + (np_ - clustered);
+  int64_t total_ctas = (int64_t)clustered * ctas + (np_ - clustered);
   const int slot_values = k == 1 ? Slot<1>::kSize : k == 6 ? Slot<6>::kSize : Slot<8>::kSize;
   const size_t tsize = 8;  // FP64-sized: the mixed path ends with an FP64 polish
-  Planner pl;
   auto plan = [&](auto& A) {
     struct Ptrs {
       double *ext, *intr, *pts, *ext2, *intr2, *pts2, *scale_p;
@@ -1541,9 +1540,22 @@ gbba_status solve_batched_impl(gbba_handle* h, const gbba_problem* probs, int32_
     q.pt_s = A.template take<uint32_t>(to);
     return q;
   };
-  plan(pl);
   h->arena.reset();
-  h->arena.reserve(pl.used + 4096);
+  auto reserve = [&]() {
+    Planner pl;
+    plan(pl);
+    h->arena.reserve(pl.used + 4096);
+  };
+  try {
+    reserve();
+  } catch (const Error& e) {
+    // every CTA of a cluster has scratch of its own: one CTA a window needs the least
+    if (e.status != GBBA_ERROR_OUT_OF_MEMORY || clustered == 0) throw;
+    cudaGetLastError();  // the failed allocation's
+    clustered = 0;
+    total_ctas = np_;
+    reserve();
+  }
   auto q = plan(h->arena);
   // parameters and observations, packed
   auto size_e = [&](int i) { return 48 * (size_t)probs[i].num_cameras; };
