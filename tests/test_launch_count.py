@@ -9,15 +9,18 @@ pytestmark = pytest.mark.gpu
 
 def kernels(handle, abi, sc, opts):
     import torch
-    hp = abi.HostProblem(sc)
-    torch.cuda.synchronize()
-    before = handle.lib.gbba_launch_count(handle.h)
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        s = handle.solve(hp, opts)
+    for _ in range(4):  # (a process's first trace may come back empty)
+        hp = abi.HostProblem(sc)
         torch.cuda.synchronize()
-    traced = sum(1 for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA
-                 and not e.name.lower().startswith(("memcpy", "memset")))
-    return s, handle.lib.gbba_launch_count(handle.h) - before, traced
+        before = handle.lib.gbba_launch_count(handle.h)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            s = handle.solve(hp, opts)
+            torch.cuda.synchronize()
+        traced = sum(1 for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA
+                     and not e.name.lower().startswith(("memcpy", "memset")))
+        if traced > 0:
+            return s, handle.lib.gbba_launch_count(handle.h) - before, traced
+    pytest.skip("the device gives no trace of its kernels")
 
 
 @pytest.mark.parametrize("graphs", [0, 1])
@@ -29,7 +32,6 @@ def test_iterations_count_what_they_launch(kind, graphs, handle, abi, scenes):
         sc["intrinsic_index"] = sc["intrinsic_index"] * 0
         sc["intrinsics"] = sc["intrinsics"][:1]
     assert (len(sc["observations"]) >= 16384) == (kind == "fp64 many")
-    kernels(handle, abi, sc, scenes.ba_options_for(sc, max_num_iterations=1))  # a process's first trace may be empty
     counts = []
     for n in (2, 4):
         opts = scenes.ba_options_for(sc, max_num_iterations=n, use_cuda_graphs=graphs, fp64_polish_iterations=0,
@@ -37,6 +39,6 @@ def test_iterations_count_what_they_launch(kind, graphs, handle, abi, scenes):
                                      precision=abi.PRECISION_MIXED if kind == "mixed" else abi.PRECISION_FP64)
         handle.solve(abi.HostProblem(sc), opts)  # (allocations and attributes)
         s, counted, traced = kernels(handle, abi, sc, opts)
-        assert s.num_iterations == n and s.num_successful_steps > 0 and traced > 0
+        assert s.num_iterations == n and s.num_successful_steps > 0
         counts.append((counted, traced))
     assert counts[1][0] - counts[0][0] == counts[1][1] - counts[0][1]
